@@ -233,8 +233,8 @@ int sa_amg_sweep(sa_ctx ctx, sa_amg M, int level, const void *in, void *out);
  * they solve -- their GPU memory is already claimed by another allocator (a
  * framework's caching allocator, a fixed pool), or they cannot afford the
  * device-wide synchronisation that allocating and freeing imply.  in and out
- * must be device buffers.  The fine-level sweep kernel's scratch comes from a
- * static device array sized for 262,144 rows (2 MiB, held by every GPU that
+ * must be device buffers.  The scratch of a sweep by several CTAs comes from a
+ * static device array sized for 262,144 rows (4 MiB, held by every GPU that
  * loads the library until the process exits); a level with more rows is
  * rejected with SA_ERR_ARG.  The first call on a device looks up that array's
  * address, so make the first call before any stream capture.  Every call

@@ -52,12 +52,13 @@ std::unique_ptr<DevAmg> upload_amg_int(Ctx &c, std::shared_ptr<IntHierarchy> h) 
     for (auto &m : h->P) M->P.push_back(upload_csr_i32(m));
     for (auto &m : h->R) M->R.push_back(upload_csr_i32(m));
     for (auto &m : h->U) M->U.push_back(upload_csr_i32(m));
+    std::vector<TriSource> ld;
     for (int l = 0; l < h->depth; l++) {
         const CsrI &m = h->LD[l];
         const int *hint = h->colour[l].empty() ? nullptr : h->colour[l].data();
-        M->LD.push_back(
-            upload_tri(c, m.n, m.rptr.data(), m.cind.data(), m.val.data(), VT_I32, TRI_LD, m.bit, m.dbit, hint));
+        ld.push_back(TriSource{m.n, m.rptr.data(), m.cind.data(), m.val.data(), m.bit, m.dbit, hint});
     }
+    M->LD = upload_tris(c, ld, VT_I32);
     M->nbj = h->bj.empty() || h->bj[0].empty() ? 0 : (int)h->bj[0].size() - 1;
     M->LU = upload_dense_lu(h->LUL.rptr.data(), h->LUL.cind.data(), h->LUL.val.data(), h->LUU.rptr.data(),
                             h->LUU.cind.data(), h->LUU.val.data(), h->LUL.n, VT_I32, h->LUL.bit, h->LUU.bit,
@@ -78,11 +79,13 @@ static std::unique_ptr<DevAmg> upload_amg_fp(Ctx &c, const FpHierarchy<T> &h, in
     for (auto &m : h.P) M->P.push_back(upload_csr_fp<T>(m));
     for (auto &m : h.R) M->R.push_back(upload_csr_fp<T>(m));
     for (auto &m : h.U) M->U.push_back(upload_csr_fp<T>(m));
+    std::vector<TriSource> ld;
     for (int l = 0; l < h.depth; l++) {
         const auto &m = h.LD[l];
         const int *hint = h.colour[l].empty() ? nullptr : h.colour[l].data();
-        M->LD.push_back(upload_tri(c, m.n, m.rptr.data(), m.cind.data(), m.val.data(), vt, TRI_LD, 0, 0, hint));
+        ld.push_back(TriSource{m.n, m.rptr.data(), m.cind.data(), m.val.data(), 0, 0, hint});
     }
+    M->LD = upload_tris(c, ld, vt);
     M->nbj = h.bj.empty() || h.bj[0].empty() ? 0 : (int)h.bj[0].size() - 1;
     M->LU = upload_dense_lu(h.LUL.rptr.data(), h.LUL.cind.data(), h.LUL.val.data(), h.LUU.rptr.data(),
                             h.LUU.cind.data(), h.LUU.val.data(), h.LUL.n, vt, 0, 0, 0);

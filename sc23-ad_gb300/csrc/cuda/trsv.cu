@@ -10,14 +10,14 @@
 // the integer results of the sequential loop.
 //
 // Two kernels:
-//  * k_tri_cta (coarse levels, the vector fits in shared memory): one CTA.  The
-//    result vector lives in shared memory, seeded with `in` (a row reads its own
-//    input once and then overwrites it).  Each level's row data is one 16-byte
-//    aligned block that a bulk copy (cp.async.bulk + mbarrier) brings into a
-//    byte ring in shared memory (all of it not taken by the vector) up to
-//    kSlots levels ahead, so a level costs shared memory traffic and one block
-//    barrier.
-//  * k_tri (fine levels): one CTA per SM claims chunks of level-ordered rows
+//  * k_sweep: contiguous blocks of rows, one CTA each, the block's values in
+//    shared memory, every level's row data streamed ahead by bulk copies; one
+//    block where the vector fits one CTA's shared memory and the levels are
+//    small.  It needs every row of a block to read rows of the same or of
+//    earlier blocks.
+//  * k_tri (what k_sweep's plan cannot hold: large multicolour sweeps, whose
+//    rows also read later rows, and triangles that reach back too far for the
+//    shared memory): one CTA per SM claims chunks of level-ordered rows
 //    by ticket; a row waits only for the rows it reads.  Integer and FP32
 //    results are published as one 64-bit word {epoch, value}, so a dependency
 //    costs one L2 load; FP64 results use an epoch flag with release/acquire.
@@ -28,20 +28,21 @@
 // the last CTA, so both kernels replay from a CUDA graph.
 #include <algorithm>
 #include <cstring>
+#include <exception>
 #include <mutex>
+#include <system_error>
+#include <thread>
 #include <type_traits>
 
+#include "../host/sweep_plan.hpp"
 #include "../sagb_internal.hpp"
 #include "common.cuh"
 
 namespace sagb {
 
 constexpr int kTriThreads = 256;   // multi-CTA kernel
-constexpr int kCtaThreads = 1024;  // single-CTA kernel
 constexpr int kBatch = 4;          // dependencies read together per lane (multi-CTA)
-constexpr int kSlots = 8;          // levels in flight in the single CTA's bulk-copy ring
 constexpr size_t kSmemMax = 227 * 1024;
-constexpr size_t kCtaVecMax = 150 * 1024;  // largest shared result vector
 
 template <int VT>
 using vt_t = typename std::conditional<VT == VT_I32, int, typename std::conditional<VT == VT_F64, double, float>::type>::type;
@@ -243,200 +244,373 @@ __global__ void __launch_bounds__(kTriThreads) k_tri(TriArgs a, const void *in, 
     }
 }
 
-// ============================================================= single CTA
+// ================================================================ blocks
 //
-// Level block (host layout, 16-byte aligned, size a multiple of 16):
-//   int32 header[8] = {R, E, off_val, off_dinv, off_perm, off_rp, 0, 0}
-//   val[E] (V), dinv[R] (V), perm[R], rp[R+1] (0-based inside the block), pci[E]
+// k_sweep runs the plan of host/sweep_plan.hpp: CTA b (blocks claimed in order,
+// so the blocks it reads are running or done) keeps the values of its rows and
+// of its imports in shared memory and takes its rows level by level.
+//
+// What bounds it is the chain of dependency levels, so a step has to be short:
+// its static data (entries as shared memory offsets, inverse diagonals) are
+// copied to shared memory kSweepStage - 1 records ahead (each lane its own
+// part, so a record needs no barrier) and are in registers before the step's
+// barrier; a step is then one gather from shared memory, the products, the sum
+// over a row's lanes, the row rule, one store and the barrier of the CTA's
+// compute warps.  It has next to no branches: one warp runs alone on its
+// scheduler, where a branch costs about as much as a round of the sum.
+// A few more warps (importers) poll the published values of earlier blocks and
+// copy them into the import slots ahead of their use, so that a step waits for
+// another CTA only when this one has caught up with it.
+//
+// A row that later blocks read is published as 64-bit words {epoch, value}
+// (two of them for FP64, each with half of the value), which need no reset; the
+// words of a block's rows of one level are neighbours, so that a poll of 32 of
+// them takes few sectors (the pollers share the SM's load path with the sweep).
+//
+// Measured on one GB300 against the kernels it took the place of (one CTA with
+// a barrier of 31 warps and row data in level blocks; k_tri with two passes of
+// dependent loads a level): int sweeps of all nine levels of Poisson 128^3, 11.4
+// -> 3.1 ms (level 0, 382 dependency levels, 1.14 -> 0.23 ms; level 5, 1,112
+// levels of 22 rows of 164 entries, 1.66 -> 0.60 ms), of Poisson 181^2 1.29 ->
+// 0.32 ms (0.18-0.23 us a level), FP64 convection-diffusion 41^3 5.97 -> 1.13 ms.
+// What was slower: mbarrier-tracked bulk copies instead of the per-lane copies
+// (a try_wait and a vote a record: 0.25 instead of 0.18 us a level), records in
+// registers by plain loads (too few scoreboards to keep several records in
+// flight), lanes a row chosen per step (branches), importers that poll several
+// groups at once (their polls take the sweep's share of the load path), words
+// by row number (a poll of 32 rows took 32 sectors: level 0 0.44 ms).
+//
+// Every wait for a published value is bounded in time: it raises ST_TIMEOUT
+// when it runs out and the sweep goes on with the values there are.
+struct SweepBlock {
+    int row0, row1, imp0, imp1, grp0, grp1, steps, pad;  // rows, imports, entries of grp; barriers
+};
+struct SweepArgs {
+    int warps, importers_log, bit, dbit;  // 2^importers_log importers (several blocks)
+    const SweepBlock *blocks;  // gridDim.x of them
+    const long long *stream;   // first record of (block, warp)
+    const uint4 *data;
+    const int *imp_place, *grp;
+    unsigned long long *pk;
+    TriSync *sync;
+};
 
-template <int VT, int G, bool EXACT>
-__device__ __forceinline__ void cta_level(const unsigned char *blk, vt_t<VT> *s_out, int bit, int dbit, int warp,
-                                          int sub, int g, bool &ovf) {
-    using V = vt_t<VT>;
-    constexpr int RPW = 32 / G;
-    constexpr int NW = kCtaThreads / 32 - 1;  // the last warp issues the bulk copies
-    const int *hdr = (const int *)blk;
-    const int R = hdr[0];
-    const V *val = (const V *)(blk + hdr[2]);
-    const V *dv = (const V *)(blk + hdr[3]);
-    const int *perm = (const int *)(blk + hdr[4]);
-    const int *rp = (const int *)(blk + hdr[5]);
-    const int *pci = rp + R + 1;
-    for (int base = warp * RPW; base < R; base += NW * RPW) {
-        const int r = base + sub;
-        const bool valid = r < R;
-        acc_t<VT> t = 0;
-        int row = 0;
-        if (valid) {
-            row = perm[r];
-            const int jb = rp[r], je = rp[r + 1];
-            if (g == 0) t = acc_init<VT>(s_out[row], bit);
-            // four entries of the lane at a time: their loads are issued
-            // together, the products are taken in the lane's order
-            int j = jb + g;
-            for (; j + 3 * G < je; j += 4 * G) {
-                const int c0 = pci[j], c1 = pci[j + G], c2 = pci[j + 2 * G], c3 = pci[j + 3 * G];
-                const V v0 = val[j], v1 = val[j + G], v2 = val[j + 2 * G], v3 = val[j + 3 * G];
-                const V o0 = s_out[c0], o1 = s_out[c1], o2 = s_out[c2], o3 = s_out[c3];
-                t = acc_sub<VT, EXACT>(t, v0, o0);
-                t = acc_sub<VT, EXACT>(t, v1, o1);
-                t = acc_sub<VT, EXACT>(t, v2, o2);
-                t = acc_sub<VT, EXACT>(t, v3, o3);
-            }
-            for (; j < je; j += G) t = acc_sub<VT, EXACT>(t, val[j], s_out[pci[j]]);
+__device__ __forceinline__ void ld_relaxed_v2(const unsigned long long *p, unsigned long long &a,
+                                              unsigned long long &b) {
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_relaxed_v2(unsigned long long *p, unsigned long long a, unsigned long long b) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ int ld_acquire_cta(const int *p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_cta(int *p, int v) {
+    asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
+}
+
+// a published row as read: its words, whether they are of this epoch, its value
+struct Published {
+    unsigned long long a, b;
+};
+template <int VT>
+__device__ __forceinline__ Published sweep_peek(const unsigned long long *pk, int row) {
+    Published w{0ull, 0ull};
+    if constexpr (VT == VT_F64) ld_relaxed_v2(pk + 2 * (size_t)row, w.a, w.b);
+    else w.a = ld_relaxed_u64(pk + row);
+    return w;
+}
+template <int VT>
+__device__ __forceinline__ bool sweep_ready(const Published &w, unsigned ep) {
+    return (unsigned)(w.a >> 32) == ep && (VT != VT_F64 || (unsigned)(w.b >> 32) == ep);
+}
+template <int VT>
+__device__ __forceinline__ vt_t<VT> sweep_value(const Published &w) {
+    if constexpr (VT == VT_F64) return __hiloint2double((int)(unsigned)w.b, (int)(unsigned)w.a);
+    else if constexpr (VT == VT_I32) return (int)(unsigned)w.a;
+    else return __uint_as_float((unsigned)w.a);
+}
+template <int VT>
+__device__ __forceinline__ void sweep_publish(unsigned long long *pk, int row, unsigned ep, vt_t<VT> v) {
+    const unsigned long long hi = (unsigned long long)ep << 32;
+    if constexpr (VT == VT_F64)
+        st_relaxed_v2(pk + 2 * (size_t)row, hi | (unsigned)__double2loint(v), hi | (unsigned)__double2hiint(v));
+    else if constexpr (VT == VT_I32)
+        st_relaxed_u64(pk + row, hi | (unsigned)v);
+    else
+        st_relaxed_u64(pk + row, hi | __float_as_uint(v));
+}
+
+// the sum of 2^LG neighbouring lanes; 32 lanes of 64-bit integers as three
+// REDUX of 22, 21 and 21 bits (their sums fit 32 bits)
+template <int VT, int LG>
+__device__ __forceinline__ acc_t<VT> sweep_sum(acc_t<VT> t) {
+    if constexpr (VT == VT_I32 && LG == 5) {
+        const unsigned long long u = (unsigned long long)t;
+        const unsigned a = __reduce_add_sync(0xffffffffu, (unsigned)u & 0x3fffffu);
+        const unsigned b = __reduce_add_sync(0xffffffffu, (unsigned)(u >> 22) & 0x1fffffu);
+        const unsigned c = __reduce_add_sync(0xffffffffu, (unsigned)(u >> 43));
+        return (long long)((unsigned long long)a + ((unsigned long long)b << 22) + ((unsigned long long)c << 43));
+    } else {
+#pragma unroll
+        for (int o = 1 << LG >> 1; o > 0; o >>= 1) {
+            if constexpr (VT == VT_I32) t = wadd(t, shfl_xor(t, o));
+            else t += shfl_xor(t, o);
         }
-        t = acc_reduce<VT>(t, G);
-        if (valid && g == 0) s_out[row] = acc_finish<VT>(t, dv[r], bit, dbit, ovf);
+        return t;
     }
 }
 
-// Shared memory of the single-CTA kernel: the result vector, a byte ring for
-// the level blocks, kSlots mbarriers, the ring position of each level in
-// flight, the block offsets and the rows of each level.  The first lane of
-// the last warp (the producer; that warp computes no rows, so issuing copies
-// never delays a level) places every block contiguously in the ring, in level
-// order (at the write position, or at the ring's start when the end has no
-// room), as soon as the ring has room and fewer than kSlots levels are in
-// flight; a block larger than the whole ring is read from global memory
-// instead.  Level d is always placed by the time the CTA reaches it: the
-// producer places it right after the barrier of level d-1 at the latest, when
-// every earlier level has been consumed and the ring is empty.
-//
-// (A variant without the barrier per level, each row waiting on done bits of
-// the rows it reads, ran about twice as slow on the coarse levels of Poisson
-// 128^3: the waiting rows' shared-memory polling slowed the rows being
-// computed more than the barrier costs.)
-template <int VT, int G, bool EXACT>
-__global__ void __launch_bounds__(kCtaThreads, 1)
-k_tri_cta(const unsigned char *__restrict__ blocks, const unsigned *__restrict__ blk_off, int nlev, int n,
-          int bit, int dbit, int ring_bytes, const void *in_, void *out_, unsigned *flags) {
-    using V = vt_t<VT>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V *s_out = (V *)smem_raw;
-    const size_t vec_bytes = ((size_t)n * sizeof(V) + 15) & ~(size_t)15;
-    unsigned char *ring = smem_raw + vec_bytes;
-    unsigned long long *bar = (unsigned long long *)(ring + ring_bytes);
-    unsigned *s_pos = (unsigned *)(bar + kSlots);  // ring offset of each level in flight
-    unsigned *s_off = s_pos + kSlots;              // block offsets in 16-byte units
-    const unsigned *s_rows = s_off + nlev + 1;     // rows of each level
-    const V *in = (const V *)in_;
-    V *out = (V *)out_;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane % G, sub = lane / G;
-    constexpr int kProducerWarp = kCtaThreads / 32 - 1;
-    const bool compute = warp != kProducerWarp;
-    const bool producer = warp == kProducerWarp && lane == 0;
-    bool ovf = false;
+// shared memory by 32-bit address (volatile: they keep their order around the
+// barriers)
+template <typename V>
+__device__ __forceinline__ V lds_val(unsigned a) {
+    V v;
+    if constexpr (sizeof(V) == 8) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    else if constexpr (std::is_same<V, float>::value) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    else asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+// (a store that is skipped where `no` is not zero)
+template <typename V>
+__device__ __forceinline__ void sts_unless(unsigned no, unsigned a, V v) {
+#define SAGB_STS(TYPE, C)                                                                                     \
+    asm volatile("{\n .reg .pred p;\n setp.eq.u32 p, %2, 0;\n @p st.shared." TYPE " [%0], %1;\n}\n" ::"r"(a), \
+                 C(v), "r"(no)                                                                                \
+                 : "memory")
+    if constexpr (sizeof(V) == 8) SAGB_STS("f64", "d");
+    else if constexpr (std::is_same<V, float>::value) SAGB_STS("f32", "f");
+    else SAGB_STS("s32", "r");
+#undef SAGB_STS
+}
+__device__ __forceinline__ uint4 lds_quad(unsigned a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+// 16 bytes to this lane's own part of shared memory, counted by copy groups
+__device__ __forceinline__ void copy_quad(unsigned dst, const uint4 *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-    if (producer) {
-        for (int s = 0; s < kSlots; s++) mbar_init(bar + s, 1);
-        fence_mbar_init();
+constexpr int kSweepThreads = 32 * (kSweepMaxWarps + kSweepImporters);
+
+template <int VT, bool EXACT, int LG, int E>
+__global__ void __launch_bounds__(kSweepThreads, 1)
+k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
+    using V = vt_t<VT>;
+    constexpr int Q = 1 + E + (VT == VT_F64);  // quads of a record
+    constexpr unsigned RB = Q * 512;           // its bytes
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int W = a.warps, IM = 1 << a.importers_log;
+    int *s_misc = (int *)smem_raw;  // block, epoch
+    int *s_done = s_misc + 4;       // import groups each importer has filled
+    unsigned char *stage = smem_raw + 128;
+    V *slots = (V *)(stage + W * kSweepStage * RB);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool many = gridDim.x > 1;
+    if (threadIdx.x == 0) {
+        s_misc[0] = many ? (int)atomicAdd(&a.sync->ticket, 1u) : 0;
+        s_misc[1] = many ? (int)(ld_acquire_u32(&a.sync->epoch) + 1) : 0;
     }
-    for (int i = threadIdx.x; i < n; i += kCtaThreads) s_out[i] = in[i];
-    for (int i = threadIdx.x; i <= 2 * nlev; i += kCtaThreads) s_off[i] = __ldg(blk_off + i);
+    if (threadIdx.x < kSweepImporters) s_done[threadIdx.x] = 0;
     __syncthreads();
-    auto bytes_of = [&](int d) { return (s_off[d + 1] - s_off[d]) * 16u; };
-    auto staged = [&](int d) { return bytes_of(d) <= (unsigned)ring_bytes; };
-    // the producer's ring state: levels [consumed, issued) are in flight; the
-    // nst staged ones among them occupy [lo, head), wrapped once when head <= lo
-    int issued = 0, nst = 0;
-    unsigned lo = 0, head = 0;
-    auto issue_more = [&](int consumed) {  // producer only
-        while (issued < nlev && issued - consumed < kSlots) {
-            const int d = issued;
-            if (staged(d)) {
-                const unsigned b = bytes_of(d);
-                unsigned pos;
-                if (nst == 0) {
-                    pos = 0;
-                    lo = 0;
-                } else if (head > lo) {  // [lo, head): room at the end, else at the start
-                    if (b <= (unsigned)ring_bytes - head) pos = head;
-                    else if (b <= lo) pos = 0;
-                    else break;
-                } else {  // [lo, ring) and [0, head): room between head and lo
-                    if (b <= lo - head) pos = head;
-                    else break;
-                }
-                head = pos + b;
-                nst++;
-                const int s = d % kSlots;
-                // the region's previous readers passed the level barrier
-                // before this copy is issued (no proxy fence is needed for a
-                // bulk copy into memory that generic loads only read)
-                s_pos[s] = pos;  // published to the waiting threads by the arrive below
-                mbar_expect_tx(bar + s, b);
-                bulk_g2s(ring + pos, blocks + (size_t)s_off[d] * 16, b, bar + s);
-            }
-            issued++;
-        }
-    };
-    if (producer) issue_more(0);
-    unsigned phase = 0;  // bit s: parity of slot s's next completion
-    int stuck = -1;      // level whose copy did not arrive in time
-    for (int d = 0; d < nlev; d++) {
-        const bool st = staged(d);
-        const int s = d % kSlots;
-        const unsigned char *blk = blocks + (size_t)s_off[d] * 16;
-        bool timed_out = false;
-        // a warp with no row in this level neither waits for its block nor
-        // reads it (it only keeps the slot parities)
-        constexpr int kRowsPerWarp = 32 / G;
-        const bool mine = compute && warp * kRowsPerWarp < (int)s_rows[d];
-        if (st && !mine) {
-            phase ^= 1u << s;
-        } else if (st) {
-            // bounded wait for the bulk copy of this level
-            const unsigned par = (phase >> s) & 1u;
-            if (!mbar_try_wait(bar + s, par)) {
-                const unsigned long long t0 = globaltimer_ns();
-                while (!mbar_try_wait(bar + s, par)) {
-                    if (globaltimer_ns() - t0 > kSpinLimitNs) {
-                        timed_out = true;
-                        break;
+    const int blk = s_misc[0];
+    const unsigned ep = (unsigned)s_misc[1];
+    const SweepBlock B = a.blocks[blk];
+    const int rows = B.row1 - B.row0, nimp = B.imp1 - B.imp0;
+
+    if (warp >= W) {
+        // ------------------------------------------------------ importers
+        const int w = warp - W, groups = B.grp1 - B.grp0 - 1;
+        V *sv = slots + rows;
+        // the place of this lane's row in group k
+        auto import_of = [&](int k, int &idx) {
+            if (k >= groups) return -1;
+            idx = __ldg(a.grp + B.grp0 + k) + lane;
+            return idx < __ldg(a.grp + B.grp0 + k + 1) ? __ldg(a.imp_place + B.imp0 + idx) : -1;
+        };
+        // places two groups ahead, a first look at the values one ahead: a
+        // group whose values are there already costs no round trip of its own
+        int idx0 = 0, idx1 = 0, filled = 0;
+        int row0 = import_of(w, idx0), row1 = import_of(w + IM, idx1);
+        Published v0{0ull, 0ull};
+        if (row0 >= 0) v0 = sweep_peek<VT>(a.pk, row0);
+        for (int k = w; k < groups; k += IM) {
+            Published v1{0ull, 0ull};
+            if (row1 >= 0) v1 = sweep_peek<VT>(a.pk, row1);
+            int idx2 = 0;
+            const int row2 = import_of(k + 2 * IM, idx2);
+            if (row0 >= 0) {
+                if (!sweep_ready<VT>(v0, ep)) {
+                    const unsigned long long t0 = globaltimer_ns();
+                    for (unsigned it = 1;; it++) {
+                        v0 = sweep_peek<VT>(a.pk, row0);
+                        if (sweep_ready<VT>(v0, ep)) break;
+                        if ((it & 255u) == 0) {
+                            if (globaltimer_ns() - t0 > kSpinLimitNs) {
+                                atomicOr(flags, ST_TIMEOUT);
+                                break;
+                            }
+                            if (aborted(flags)) break;
+                        }
                     }
                 }
+                sv[idx0] = sweep_value<VT>(v0);
             }
-            phase ^= 1u << s;
-            blk = ring + s_pos[s];
+            idx0 = idx1;
+            row0 = row1;
+            v0 = v1;
+            idx1 = idx2;
+            row1 = row2;
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) st_release_cta(s_done + w, ++filled);
         }
-        if (mine && !timed_out) cta_level<VT, G, EXACT>(blk, s_out, bit, dbit, warp, sub, g, ovf);
-        // one barrier per level: results visible, the level's ring space free
-        if (__syncthreads_or(timed_out)) {
-            stuck = d;
-            break;
-        }
-        if (producer) {
-            if (st && --nst > 0) {
-                for (int e = d + 1; e < issued; e++)
-                    if (staged(e)) {
-                        lo = s_pos[e % kSlots];
-                        break;
-                    }
-            }
-            issue_more(d + 1);
-        }
-    }
-    if (stuck >= 0) {
-        // report, then wait (bounded) for the copies this CTA still has in
-        // flight before its shared memory goes away
-        if (producer) {
-            atomicOr(flags, ST_TIMEOUT);
-            const unsigned long long t0 = globaltimer_ns();
-            for (int dd = stuck; dd < issued; dd++) {
-                if (!staged(dd)) continue;
-                const int s = dd % kSlots;
-                // the stuck level's wait already flipped its parity bit
-                const unsigned par = ((phase >> s) & 1u) ^ (dd == stuck ? 1u : 0u);
-                while (!mbar_try_wait(bar + s, par) && globaltimer_ns() - t0 < kSpinLimitNs) {
-                }
-            }
-        }
-        __syncthreads();
         return;
     }
-    for (int i = threadIdx.x; i < n; i += kCtaThreads) out[i] = s_out[i];
+
+    // ------------------------------------------------------------ compute
+    const long long r0 = a.stream[(size_t)blk * W + warp];
+    const int nrec = (int)(a.stream[(size_t)blk * W + warp + 1] - r0);
+    // (the streams are padded: copies past a warp's last record stay inside)
+    const uint4 *src = a.data + (size_t)r0 * (Q * 32) + lane;
+    const unsigned mine = smem_addr(stage) + warp * (kSweepStage * RB) + lane * 16;
+    auto copy = [&](unsigned at) {
+#pragma unroll
+        for (int q = 0; q < Q; q++) copy_quad(mine + at + q * 512, src + q * 32);
+        copy_commit();
+        src += Q * 32;
+    };
+#pragma unroll
+    for (int k = 0; k < kSweepStage - 1; k++) copy(k * RB);
+    const unsigned char *ahead = (const unsigned char *)(a.data + (size_t)r0 * (Q * 32)) + lane * 128;
+    if (lane < 4 * Q)
+        for (int k = kSweepStage; k < kSweepAhead; k++) prefetch_l2(ahead + (size_t)k * RB);
+    ahead += (size_t)kSweepAhead * RB;
+    {
+        const V *in = (const V *)in_ + B.row0;
+#pragma unroll 8
+        for (int i = threadIdx.x; i < rows; i += W * 32) slots[i] = in[i];
+        if (threadIdx.x < 2) slots[rows + nimp + threadIdx.x] = V(0);
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+    const unsigned sl = smem_addr(slots);
+    int step = 0, need = 0;  // barriers passed, import groups needed
+    bool ovf = false, fresh = true;
+    acc_t<VT> t = 0;
+    unsigned to = (kSweepStage - 1) * RB, from = RB;  // where the next copy goes and the next record is
+    // one record, in registers in r; the next one is brought into n
+    auto record = [&](const uint4(&r)[Q], uint4(&n)[Q], bool odd) {
+        const unsigned c = r[0].x;
+        for (unsigned k = c >> 18 & 127u; k > 0; k--) {
+            asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+            step++;
+        }
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p bar.sync 1, %1;\n}\n" ::"r"(c & (1u << 17)), "r"(W * 32)
+                     : "memory");
+        step += (int)(c >> 17 & 1u);
+        if (c >> 25) {
+            // importer w has filled its groups w, w + IM, ...
+            need += (int)(c >> 25);
+            const int w = lane & (IM - 1), want = (need - w + IM - 1) >> a.importers_log;
+            if (ld_acquire_cta(s_done + w) < want) {
+                const unsigned long long t0 = globaltimer_ns();
+                while (ld_acquire_cta(s_done + w) < want)
+                    if (globaltimer_ns() - t0 > 2 * kSpinLimitNs) {
+                        atomicOr(flags, ST_TIMEOUT);
+                        break;
+                    }
+            }
+            __syncwarp();
+        }
+        V x[2 * E];
+#pragma unroll
+        for (int h = 0; h < 2 * E; h++) {
+            if constexpr (VT == VT_F64) {
+                const uint4 &o = r[1 + E];
+                const unsigned w = h / 2 == 0 ? o.x : h / 2 == 1 ? o.y : h / 2 == 2 ? o.z : o.w;
+                x[h] = lds_val<V>(sl + (h & 1 ? w >> 16 : w & 0xffffu) * 8);
+            } else {
+                x[h] = lds_val<V>(sl + (h & 1 ? r[1 + h / 2].z : r[1 + h / 2].x));
+            }
+        }
+        const unsigned row = sl + (c & 0xffffu) * (unsigned)sizeof(V);
+        const V own = lds_val<V>(row);
+        // the record kSweepStage - 1 ahead goes where the last one was
+        copy(to);
+        to = to == (kSweepStage - 1) * RB ? 0 : to + RB;
+        if (odd) {  // two records' lines
+            if (lane < 8 * Q) prefetch_l2(ahead);
+            ahead += 2 * RB;
+        }
+        copy_wait<kSweepStage - 2>();
+#pragma unroll
+        for (int q = 0; q < Q; q++) n[q] = lds_quad(mine + from + q * 512);
+        from = from == (kSweepStage - 1) * RB ? 0 : from + RB;
+        const bool more = c & (1u << 16);  // the row goes on
+        acc_t<VT> s = t, s2 = 0;  // (two chains where the order is free)
+        if constexpr (VT != VT_I32 && LG == 0) s = fresh ? own : t;  // one lane a row: its sum in its order
+#pragma unroll
+        for (int h = 0; h < 2 * E; h++) {
+            const uint4 &v = r[1 + h / 2];
+            acc_t<VT> &sum = h < E || EXACT ? s : s2;
+            if constexpr (VT == VT_I32)  // the products, subtracted at the end
+                sum = wadd(sum, (long long)(int)(h & 1 ? v.w : v.y) * (long long)x[h]);
+            else if constexpr (VT == VT_F64)
+                sum = acc_sub<VT, EXACT>(sum, h & 1 ? __hiloint2double((int)v.w, (int)v.z) : __hiloint2double((int)v.y, (int)v.x), x[h]);
+            else
+                sum = acc_sub<VT, EXACT>(sum, __uint_as_float(h & 1 ? v.w : v.y), x[h]);
+        }
+        if constexpr (VT == VT_I32) s = wadd(s, s2);
+        else if constexpr (!EXACT) s += s2;
+        t = more ? s : acc_t<VT>(0);
+        fresh = !more;
+        s = sweep_sum<VT, LG>(s);
+        V dinv;
+        if constexpr (VT == VT_F64) dinv = __hiloint2double((int)r[0].w, (int)r[0].z);
+        else if constexpr (VT == VT_I32) dinv = (int)r[0].z;
+        else dinv = __uint_as_float(r[0].z);
+        if constexpr (VT == VT_I32) s = wsub(wshl((long long)own, a.bit), s);
+        else if constexpr (LG > 0) s += own;
+        // every lane of a row has its result and stores it
+        const V v = acc_finish<VT>(s, dinv, a.bit, a.dbit, ovf);
+        sts_unless<V>(c & (1u << 16), row, v);
+        if ((int)r[0].y >= 0) sweep_publish<VT>(a.pk, (int)r[0].y, ep, v);
+    };
+    uint4 ra[Q], rb[Q];
+    copy_wait<kSweepStage - 2>();
+#pragma unroll
+    for (int q = 0; q < Q; q++) ra[q] = lds_quad(mine + q * 512);
+    for (int i = 0; i < nrec; i += 2) {
+        record(ra, rb, false);
+        if (i + 1 < nrec) record(rb, ra, true);
+    }
+    copy_wait<0>();
+    for (; step < B.steps; step++) asm volatile("bar.sync 1, %0;" ::"r"(W * 32) : "memory");
+    // the block's values are complete
+    V *out = (V *)out_ + B.row0;
+    for (int i = threadIdx.x; i < rows; i += W * 32) out[i] = slots[i];
     if (ovf) atomicOr(flags, ST_OVERFLOW);
+    if (many && threadIdx.x == 0) {
+        // this CTA's importers are done: its warps waited for every import
+        __threadfence();
+        const unsigned d = atomicAdd(&a.sync->done, 1u);
+        if (d == gridDim.x - 1) {
+            a.sync->ticket = 0;
+            a.sync->done = 0;
+            __threadfence();
+            st_release_u32(&a.sync->epoch, ep);
+        }
+    }
 }
 
 // ================================================================ upload
@@ -451,16 +625,17 @@ void DevTri::release() {
     dfree(sub_bound);
     dfree(pk);
     dfree(flag);
-    dfree(sync);
+    if (!blocks) dfree(sync);  // (a sweep by blocks: behind pk; its small arrays: behind blocks)
     dfree(blocks);
-    dfree(blk_off);
+    dfree(data);
     perm = prp = pci = chunk_lv = sub_bound = nullptr;
     pval = dinv = nullptr;
     pk = nullptr;
     flag = nullptr;
     sync = nullptr;
-    blocks = nullptr;
-    blk_off = nullptr;
+    blocks = data = nullptr;
+    stream = nullptr;
+    imp_place = grp = nullptr;
 }
 
 template <typename T>
@@ -472,133 +647,176 @@ static void gather_vals(const TriSchedule &s, const T *vals, std::vector<T> &pv,
         if (s.diag_src[p] >= 0) dv[p] = vals[s.diag_src[p]];
 }
 
-static size_t up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
-// one block per level (see the layout above k_tri_cta)
-template <typename T>
-static void build_blocks(const TriSchedule &s, const std::vector<T> &pv, const std::vector<T> &dv,
-                         std::vector<unsigned char> &blob, std::vector<long long> &off) {
-    off.assign(s.nlev + 1, 0);
-    blob.clear();
-    for (int l = 0; l < s.nlev; l++) {
-        const int p0 = s.lvl_ptr[l], p1 = s.lvl_ptr[l + 1];
-        const int R = p1 - p0;
-        const int e0 = s.prp[p0], e1 = s.prp[p1];
-        const int E = e1 - e0;
-        const size_t o_val = 32;
-        const size_t o_dinv = up(o_val + sizeof(T) * E, 8);
-        const size_t o_perm = up(o_dinv + sizeof(T) * R, 4);
-        const size_t o_rp = o_perm + 4 * (size_t)R;
-        const size_t o_pci = o_rp + 4 * (size_t)(R + 1);
-        const size_t size = up(o_pci + 4 * (size_t)E, 16);
-        const size_t base = blob.size();
-        blob.resize(base + size, 0);
-        unsigned char *b = blob.data() + base;
-        int hdr[8] = {R, E, (int)o_val, (int)o_dinv, (int)o_perm, (int)o_rp, 0, 0};
-        memcpy(b, hdr, sizeof hdr);
-        memcpy(b + o_val, pv.data() + e0, sizeof(T) * E);
-        memcpy(b + o_dinv, dv.data() + p0, sizeof(T) * R);
-        memcpy(b + o_perm, s.perm.data() + p0, 4 * (size_t)R);
-        int *rp = (int *)(b + o_rp);
-        for (int r = 0; r <= R; r++) rp[r] = s.prp[p0 + r] - e0;
-        memcpy(b + o_pci, s.pci.data() + e0, 4 * (size_t)E);
-        off[l + 1] = (long long)blob.size();
-    }
-}
-
 static int pow2_at_least(double x) {
     int g = 1;
     while (g < 32 && g < x) g <<= 1;
     return g;
 }
 
-DevTri upload_tri(const Ctx &c, int n, const int *rptr, const int *cind, const void *vals, int vt, int kind,
-                  int bit, int dbit, const int *level_hint) {
-    if (kind != TRI_LD) throw CudaError{"only LD sweeps are uploaded as sparse triangles"};
+static SweepPlan plan_tri(const Ctx &c, const TriSource &t, int vt) {
+    SweepLimits lim;
+    lim.sms = c.num_sms;
+    lim.smem = (int)kSmemMax;
+    lim.integer = vt == VT_I32;
+    lim.one_lane = vt != VT_I32 && c.fp_exact;  // sequential order inside a row
+    return build_sweep_plan(t.rptr, t.cind, t.vals, (int)vt_size(vt), t.n, lim, t.level_hint);
+}
+
+static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const SweepPlan &p) {
+    const int n = src.n, *rptr = src.rptr, *cind = src.cind;
+    const void *vals = src.vals;
     DevTri d;
     d.n = n;
-    d.kind = kind;
+    d.kind = TRI_LD;
     d.vt = vt;
-    d.bit = bit;
-    d.dbit = dbit;
-    const int64_t nnz = n ? rptr[n] : 0;
-    const double avg = n ? (double)(nnz - n) / n : 0.0;
-    const size_t es = vt_size(vt);
-    const size_t vec_bytes = up((size_t)n * es, 16);
-    d.one_cta = vec_bytes <= kCtaVecMax;
-    int G = pow2_at_least(avg / (d.one_cta ? 4 : kBatch));
-    if (vt != VT_I32 && c.fp_exact) G = 1;  // sequential order inside a row
+    d.bit = src.bit;
+    d.dbit = src.dbit;
+    d.nlev = p.nlev;
+    d.max_level_rows = p.max_level_rows;
+    d.nnz_off = p.nnz_off;
+    if (p.ok()) {
+        d.grid = p.blocks;
+        d.warps = p.warps;
+        d.importers = p.importers;
+        d.lg = p.lg;
+        d.lines = p.lines;
+        // the small arrays in one buffer (blocks, streams, imports, groups), the
+        // records in another
+        std::vector<SweepBlock> bl(p.blocks);
+        for (int b = 0; b < p.blocks; b++)
+            bl[b] = SweepBlock{p.row0[b], p.row0[b + 1], p.imp_ptr[b], p.imp_ptr[b + 1], p.grp_ptr[b], p.grp_ptr[b + 1], p.steps[b], 0};
+        std::vector<unsigned char> small;
+        auto put = [&](const void *v, size_t bytes) {
+            const size_t at = (small.size() + 15) / 16 * 16;
+            small.resize(at + bytes + 16);
+            if (bytes) memcpy(small.data() + at, v, bytes);
+            return at;
+        };
+        const size_t o_bl = put(bl.data(), bl.size() * sizeof(SweepBlock)), o_st = put(p.stream.data(), p.stream.size() * 8),
+                     o_im = put(p.imp_place.data(), p.imp_place.size() * 4), o_gr = put(p.grp.data(), p.grp.size() * 4);
+        unsigned char *base = dupload(small);
+        d.blocks = base + o_bl;
+        d.stream = (long long *)(base + o_st);
+        d.imp_place = (int *)(base + o_im);
+        d.grp = (int *)(base + o_gr);
+        const size_t rec = (size_t)p.quads * 512, bytes = (size_t)p.stream.back() * rec, pad = (kSweepAhead + 4) * rec;
+        d.data = dmalloc(bytes + pad);
+        SAGB_CUDA(cudaMemset((unsigned char *)d.data + bytes, 0, pad));
+        SAGB_CUDA(cudaMemcpy(d.data, p.data.get(), bytes, cudaMemcpyHostToDevice));
+        d.smem = sweep_fixed_smem(p.warps, p.quads) + (size_t)p.max_slots * vt_size(vt);
+        if (p.blocks > 1) {
+            const size_t words = (size_t)n * (vt == VT_F64 ? 2 : 1), all = sizeof(unsigned long long) * words + sizeof(TriSync);
+            d.pk = (unsigned long long *)dmalloc(all);
+            SAGB_CUDA(cudaMemset(d.pk, 0, all));
+            d.sync = (TriSync *)(d.pk + words);
+        }
+        return d;
+    }
+    const double avg = n ? (double)d.nnz_off / n : 0.0;
+    const int G = vt != VT_I32 && c.fp_exact ? 1 : pow2_at_least(avg / kBatch);  // (sequential order inside a row)
     d.group = G;
     const int rows_per_chunk = 2 * kTriThreads / G;
-    TriSchedule s = build_tri_schedule(rptr, cind, n, kind, rows_per_chunk, 1 << 20, level_hint);
+    TriSchedule s = build_tri_schedule(rptr, cind, n, TRI_LD, rows_per_chunk, 1 << 20, src.level_hint);
     d.nlev = s.nlev;
     d.max_level_rows = s.max_level_rows;
     d.nnz_off = (int64_t)s.pci.size();
     d.nchunks = s.nchunks();
-    std::vector<unsigned char> blob;
-    std::vector<long long> off;
     auto put_vals = [&](auto tag) {
         using T = decltype(tag);
         std::vector<T> pv, dv;
         gather_vals(s, (const T *)vals, pv, dv);
-        if (d.one_cta) {
-            build_blocks(s, pv, dv, blob, off);
-        } else {
-            d.pval = pv.empty() ? dmalloc(16) : (void *)dupload(pv);
-            d.dinv = dupload(dv);
-        }
+        d.pval = pv.empty() ? dmalloc(16) : (void *)dupload(pv);
+        d.dinv = dupload(dv);
     };
     if (vt == VT_I32) put_vals(int32_t());
     else if (vt == VT_F64) put_vals(double());
     else put_vals(float());
-    if (d.one_cta) {
-        d.blocks = blob.empty() ? (unsigned char *)dmalloc(16) : dupload(blob);
-        // block offsets in 16-byte units (nlev + 1), then the rows of each level (nlev)
-        std::vector<unsigned> off16(off.size() + s.nlev);
-        for (size_t i = 0; i < off.size(); i++) off16[i] = (unsigned)(off[i] / 16);
-        for (int l = 0; l < s.nlev; l++) off16[off.size() + l] = (unsigned)(s.lvl_ptr[l + 1] - s.lvl_ptr[l]);
-        d.blk_off = dupload(off16);
-        const size_t offs_bytes = up(4 * (2 * (size_t)s.nlev + 1), 16);
-        const size_t slot_bytes = 8 * kSlots + 4 * kSlots;  // mbarriers and ring positions
-        if (vec_bytes + offs_bytes + slot_bytes + 4096 > kSmemMax)
-            throw CudaError{"sweep schedule too large for the single-CTA kernel"};
-        d.stage_bytes = (int)((kSmemMax - vec_bytes - offs_bytes - slot_bytes) / 16 * 16);
-        d.cta_smem = vec_bytes + (size_t)d.stage_bytes + slot_bytes + offs_bytes;
+    d.perm = dupload(s.perm);
+    d.prp = dupload(s.prp);
+    d.pci = s.pci.empty() ? (int *)dmalloc(16) : dupload(s.pci);
+    d.chunk_lv = dupload(s.chunk_lv);
+    d.sub_bound = dupload(s.sub_bound);
+    if (vt == VT_F64) {
+        d.flag = (unsigned *)dmalloc(sizeof(unsigned) * std::max(n, 1));
+        SAGB_CUDA(cudaMemset(d.flag, 0, sizeof(unsigned) * std::max(n, 1)));
     } else {
-        d.perm = dupload(s.perm);
-        d.prp = dupload(s.prp);
-        d.pci = s.pci.empty() ? (int *)dmalloc(16) : dupload(s.pci);
-        d.chunk_lv = dupload(s.chunk_lv);
-        d.sub_bound = dupload(s.sub_bound);
-        if (vt == VT_F64) {
-            d.flag = (unsigned *)dmalloc(sizeof(unsigned) * std::max(n, 1));
-            SAGB_CUDA(cudaMemset(d.flag, 0, sizeof(unsigned) * std::max(n, 1)));
-        } else {
-            d.pk = (unsigned long long *)dmalloc(sizeof(unsigned long long) * std::max(n, 1));
-            SAGB_CUDA(cudaMemset(d.pk, 0, sizeof(unsigned long long) * std::max(n, 1)));
-        }
-        d.sync = (TriSync *)dmalloc(sizeof(TriSync));
-        SAGB_CUDA(cudaMemset(d.sync, 0, sizeof(TriSync)));
-        d.grid = std::max(1, std::min(d.nchunks, c.num_sms));
+        d.pk = (unsigned long long *)dmalloc(sizeof(unsigned long long) * std::max(n, 1));
+        SAGB_CUDA(cudaMemset(d.pk, 0, sizeof(unsigned long long) * std::max(n, 1)));
     }
+    d.sync = (TriSync *)dmalloc(sizeof(TriSync));
+    SAGB_CUDA(cudaMemset(d.sync, 0, sizeof(TriSync)));
+    d.grid = std::max(1, std::min(d.nchunks, c.num_sms));
     return d;
+}
+
+std::vector<DevTri> upload_tris(const Ctx &c, const std::vector<TriSource> &src, int vt) {
+    const int n = (int)src.size();
+    std::vector<SweepPlan> plans(n);
+    std::vector<std::exception_ptr> failed(n);
+    auto plan = [&](int k) {
+        try {
+            plans[k] = plan_tri(c, src[k], vt);
+        } catch (...) {
+            failed[k] = std::current_exception();
+        }
+    };
+    std::vector<std::thread> pool;
+    pool.reserve(n);
+    for (int k = 0; k < n; k++) {
+        try {
+            pool.emplace_back(plan, k);
+        } catch (const std::system_error &) {  // no more threads to be had
+            plan(k);
+        }
+    }
+    for (auto &t : pool) t.join();
+    for (auto &f : failed)
+        if (f) std::rethrow_exception(f);
+    std::vector<DevTri> out;
+    for (int k = 0; k < n; k++) {
+        out.push_back(upload_tri(c, src[k], vt, plans[k]));
+        plans[k] = SweepPlan();
+    }
+    return out;
 }
 
 template <int VT, int G, bool EXACT>
 static void launch_tri(Ctx &c, const DevTri &T, const void *in, void *out) {
-    if (T.one_cta) {
-        k_tri_cta<VT, G, EXACT><<<1, kCtaThreads, T.cta_smem, c.stream>>>(
-            T.blocks, T.blk_off, T.nlev, T.n, T.bit, T.dbit, T.stage_bytes, in, out, c.d_flags);
-    } else {
-        TriArgs a{T.n, T.nchunks, T.bit, T.dbit, T.perm, T.prp, T.pci, T.pval, T.dinv,
-                  T.chunk_lv, T.sub_bound, T.pk, T.flag, T.sync};
-        k_tri<VT, G, EXACT><<<T.grid, kTriThreads, 0, c.stream>>>(a, in, out, c.d_flags);
-    }
+    TriArgs a{T.n, T.nchunks, T.bit, T.dbit, T.perm, T.prp, T.pci, T.pval, T.dinv,
+              T.chunk_lv, T.sub_bound, T.pk, T.flag, T.sync};
+    k_tri<VT, G, EXACT><<<T.grid, kTriThreads, 0, c.stream>>>(a, in, out, c.d_flags);
     c.launches++;
+}
+
+using SweepKernel = void (*)(SweepArgs, const void *, void *, unsigned *);
+template <int VT, bool EXACT, int LG>
+static SweepKernel sweep_kernel_of(int lines) {
+    return lines == 1 ? k_sweep<VT, EXACT, LG, 1> : lines == 2 ? k_sweep<VT, EXACT, LG, 2> : k_sweep<VT, EXACT, LG, 4>;
+}
+template <int VT, bool EXACT>
+static SweepKernel sweep_kernel(int lg, int lines) {
+    switch (lg) {
+        case 0: return sweep_kernel_of<VT, EXACT, 0>(lines);
+        case 1: return sweep_kernel_of<VT, EXACT, 1>(lines);
+        case 2: return sweep_kernel_of<VT, EXACT, 2>(lines);
+        case 3: return sweep_kernel_of<VT, EXACT, 3>(lines);
+        case 4: return sweep_kernel_of<VT, EXACT, 4>(lines);
+        default: return sweep_kernel_of<VT, EXACT, 5>(lines);
+    }
 }
 
 template <int VT, bool EXACT>
 static void tri_by_group(Ctx &c, const DevTri &T, const void *in, void *out) {
+    if (T.blocks) {
+        int ilog = 0;
+        while (2 << ilog <= T.importers) ilog++;
+        SweepArgs a{T.warps, ilog, T.bit, T.dbit, (const SweepBlock *)T.blocks, T.stream, (const uint4 *)T.data, T.imp_place,
+                    T.grp, T.pk, T.sync};
+        sweep_kernel<VT, EXACT>(T.lg, T.lines)<<<T.grid, 32 * (T.warps + T.importers), T.smem,
+                                                 c.stream>>>(a, in, out, c.d_flags);
+        c.launches++;
+        return;
+    }
     switch (T.group) {
         case 1: return launch_tri<VT, 1, EXACT>(c, T, in, out);
         case 2: return launch_tri<VT, 2, EXACT>(c, T, in, out);
@@ -628,14 +846,14 @@ void trsv(Ctx &c, const DevTri &T, const void *in, void *out) {
 // kernel needs per-row scratch (the packed {epoch, value} words and the
 // ticket/epoch block); this variant takes it from the file-scope array below
 // instead of the schedule's own allocation.  The array is sized for
-// kNoAllocRows rows (2 MiB) and every GPU that loads the library holds it
+// kNoAllocRows rows (two words each for FP64: 4 MiB) and every GPU that loads the library holds it
 // until the process exits.  All calls share it and it keeps the last call's
 // contents, so before each call the words of this level's rows and the
 // ticket, done and epoch counters are cleared (a previous call may have left
 // words of another precision there): every call starts at epoch 1 against
 // zeroed words.  Calls that overlap on the GPU race on this array.
 constexpr int kNoAllocRows = 262144;
-static __device__ __align__(256) unsigned long long g_noalloc_scratch[kNoAllocRows + 2];
+static __device__ __align__(256) unsigned long long g_noalloc_scratch[2 * kNoAllocRows + 2];
 
 static std::mutex g_noalloc_mu;
 static void *g_noalloc_addr[64];
@@ -659,15 +877,15 @@ static unsigned long long *noalloc_scratch(int device) {
 }
 
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
-    if (T.n == 0 || T.one_cta) return trsv(c, T, in, out);  // shared memory only: no scratch
+    if (T.n == 0 || (T.blocks && T.grid == 1)) return trsv(c, T, in, out);  // shared memory only: no scratch
     if (T.n > kNoAllocRows)
         throw CudaError{"level has more than 262144 rows, the limit of the no-allocation sweep"};
     unsigned long long *s = noalloc_scratch(c.device);
     DevTri U = T;  // same schedule and operator, scratch from the static array
     U.pk = s;
     U.flag = (unsigned *)s;
-    U.sync = (TriSync *)(s + kNoAllocRows);
-    SAGB_CUDA(cudaMemsetAsync(s, 0, sizeof(unsigned long long) * (size_t)T.n, c.stream));
+    U.sync = (TriSync *)(s + 2 * kNoAllocRows);
+    SAGB_CUDA(cudaMemsetAsync(s, 0, sizeof(unsigned long long) * (size_t)T.n * (T.vt == VT_F64 ? 2 : 1), c.stream));
     SAGB_CUDA(cudaMemsetAsync(U.sync, 0, sizeof(TriSync), c.stream));  // ticket, done, epoch
     if (U.vt == VT_I32) return tri_by_group<VT_I32, false>(c, U, in, out);
     if (U.vt == VT_F64) {
@@ -698,7 +916,7 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
            int bitL, int bitU, int dbitU, const void *__restrict__ in_, void *__restrict__ out_, unsigned *flags) {
     using V = vt_t<VT>;
     using T = acc_t<VT>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     T *t = (T *)smem_raw;                           // n accumulators
     V *x = (V *)(smem_raw + sizeof(T) * (size_t)n); // n solved values
     const V *L = (const V *)L_;
@@ -866,12 +1084,9 @@ static void launch_lu(Ctx &c, const DevDenseLU &LU, const void *in, void *out) {
 template <int VT, bool EXACT>
 static void cta_attrs() {
     const int mx = (int)kSmemMax;
-    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 1, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 2, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 4, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 8, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 16, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 32, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    for (int lg = 0; lg <= 5; lg++)
+        for (int lines = 1; lines <= 4; lines *= 2)
+            SAGB_CUDA(cudaFuncSetAttribute(sweep_kernel<VT, EXACT>(lg, lines), cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     SAGB_CUDA(cudaFuncSetAttribute(k_dense_lu<VT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
 }
 

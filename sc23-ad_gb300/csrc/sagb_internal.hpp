@@ -122,25 +122,33 @@ struct DevTri {
     int *perm = nullptr, *prp = nullptr, *pci = nullptr;
     void *pval = nullptr, *dinv = nullptr;
     int *chunk_lv = nullptr, *sub_bound = nullptr;
-    unsigned long long *pk = nullptr;  // packed {epoch, value} per row (int32 / f32)
+    unsigned long long *pk = nullptr;  // packed {epoch, value} per row (int32 / f32; two words per f64 row of a sweep by blocks)
     unsigned *flag = nullptr;          // ready epoch per row (f64)
     TriSync *sync = nullptr;
-    // single-CTA mode: the result vector in shared memory, each level's row
-    // data in one 16-byte aligned block fetched ahead by bulk copies
-    bool one_cta = false;
-    unsigned char *blocks = nullptr;
-    unsigned *blk_off = nullptr;       // offset of each level's block in 16-byte units (nlev + 1), then
-                                       // the rows of each level (nlev)
-    int stage_bytes = 0;               // bytes of the single-CTA kernel's bulk-copy ring
-    size_t cta_smem = 0;
+    // the sweep by blocks of rows (host/sweep_plan.hpp; blocks null: k_tri):
+    // grid CTAs of `warps` compute warps and `importers`, 2^lg lanes a row, `lines` pairs of
+    // entries a lane and record
+    void *blocks = nullptr, *data = nullptr;
+    long long *stream = nullptr;
+    int *imp_place = nullptr, *grp = nullptr;
+    int warps = 0, importers = 0, lg = 0, lines = 0;
+    size_t smem = 0;
     void release();
 };
 
-// Builds the schedule from a triangular CSR (kind: TRI_LD / TRI_L / TRI_DU) and
-// uploads it.  vals points at int32 / double / float values of the source CSR.
-// level_hint (optional): the level of each row (colours of a multicolour split).
-DevTri upload_tri(const Ctx &c, int n, const int *rptr, const int *cind, const void *vals, int vt, int kind,
-                  int bit, int dbit, const int *level_hint = nullptr);
+// One LD sweep to upload: a triangular CSR with int32 / double / float values
+// (off-diagonal entries, then D^-1 last in each row); level_hint (optional): the
+// level of each row (colours of a multicolour split).
+struct TriSource {
+    int n = 0;
+    const int *rptr = nullptr, *cind = nullptr;
+    const void *vals = nullptr;
+    int bit = 0, dbit = 0;
+    const int *level_hint = nullptr;
+};
+// Builds the sweeps' plans (all of them side by side on host threads) and
+// uploads them.
+std::vector<DevTri> upload_tris(const Ctx &c, const std::vector<TriSource> &src, int vt);
 void trsv(Ctx &c, const DevTri &T, const void *in, void *out);
 // the same sweep with its scratch in a static device array (no allocation)
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out);
