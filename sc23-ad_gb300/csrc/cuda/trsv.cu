@@ -900,15 +900,55 @@ void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
 //
 // LUflex::Solve / LU<T>::Solve (solver/lu.hpp:91-94, 30-33): ltri forward then
 // dutri backward on the coarsest operator's exact LU factors (30-45% dense at
-// these sizes), stored dense and row-major.  One CTA, 32-row panels, left
-// looking: the 32 warps first reduce each panel row against the solved part
-// (one warp per row, lanes over columns), then warp 0 solves the 32x32 diagonal
-// block with the block held in registers (shuffle broadcast of each value).
-// Integer sums are exact in any order.  In the FP sequential-order mode the
-// panel reduction runs one thread per row in column order (ascending forward,
-// descending backward), which is the reference's order.
+// these sizes), stored as 32 x 32 blocks of the triangles, 16 bytes of a row
+// together and the 32 rows of a block side by side (block_at).  Rows beyond n
+// are zero.
+//
+// k_lu_chain: one cluster of kLuCtas CTAs.  Both substitutions are one chain of
+// n rows, which a single warp walks (lane = row of the panel): it takes a
+// panel's diagonal block and the blocks of the kLuNear panels after it from shared
+// memory, and in each of 32 steps broadcasts one value by a shuffle and
+// subtracts its column from the panel and from the next ones.  What the chain
+// costs is the step's latency (integers: shift, shuffle, multiply-add); all else
+// is kept off it.  The products with the columns further back are summed by the
+// other warps of the cluster, each for its own panels, as the values come in; a
+// panel's sum is needed only kLuNear panels after the last value it takes.  Values
+// and sums travel as st.async into the other CTA's shared memory, counted by
+// one mbarrier each; a loader warp brings the chain's blocks ahead of it.
+// Integer sums wrap, so their order does not matter; FP sums are taken in
+// another order than the reference's (the sequential-order mode and factors too
+// large for the shared memory use k_dense_lu).
+// Every wait is bounded in time (ST_TIMEOUT); after one that ran out the waits
+// of that CTA no longer wait.
+// A step is 75-80 cycles for integers, 60 for FP32 and 265 for FP64, whose
+// multiply-add keeps a scheduler busy for 64.  One solve, against one CTA with
+// 32-row panels (k_dense_lu on row-major factors): int n = 512 164 -> 43 us, n =
+// 1013 338 -> 82 us, n = 1769 637 -> 142 us; FP64 n = 1872 1,520 -> 521 us; FP32
+// n = 1013 158 -> 64 us.
 
-constexpr int kLuThreads = 1024;
+constexpr int kLuThreads = 1024;   // k_dense_lu
+constexpr int kLuCtas = 8;         // k_lu_chain: CTAs of the cluster
+constexpr int kLuWarps = 8;        // and warps of each
+constexpr size_t kLuChainSmem = kSmemMax - 256;  // (the rest is static)
+constexpr int kLuSlots = 3;        // panels of the chain's blocks in shared memory
+constexpr int kLuHelpers = (kLuCtas - 1) * kLuWarps;
+// blocks after the diagonal one that the chain takes along: they cover the way of
+// a panel's values to the other CTAs and of a sum back, and cost the chain a
+// multiply-add a step.  1 / 2 / 3 of them: int n = 1769 142 / 146 / 160 us, FP32
+// n = 1013 64 / 64 / 68 us, FP64 n = 1872 521 / 653 us / -
+constexpr int kLuNear = 1;
+
+// index of element (i, c) of a block triangle: lower (column panel by column
+// panel, downwards from the diagonal) or upper (upwards from the diagonal)
+__host__ __device__ __forceinline__ size_t block_lower(int npan, int q, int p) {
+    return (size_t)p * npan - (size_t)p * (p - 1) / 2 + (q - p);
+}
+__host__ __device__ __forceinline__ size_t block_upper(int q, int p) { return (size_t)p * (p + 1) / 2 + (p - q); }
+template <typename V>
+__host__ __device__ __forceinline__ int block_at(int i, int c) {  // within a block
+    constexpr int per = 16 / (int)sizeof(V);
+    return (c / per) * (32 * per) + i * per + c % per;
+}
 
 template <int VT, bool EXACT>
 __global__ void __launch_bounds__(kLuThreads, 1)
@@ -919,12 +959,16 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T *t = (T *)smem_raw;                           // n accumulators
     V *x = (V *)(smem_raw + sizeof(T) * (size_t)n); // n solved values
-    const V *L = (const V *)L_;
-    const V *U = (const V *)U_;
     const V *dinv = (const V *)dinv_;
     const V *in = (const V *)in_;
     V *out = (V *)out_;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, npan = (n + 31) / 32;
+    auto L = [&](int i, int c) {
+        return __ldg((const V *)L_ + block_lower(npan, i >> 5, c >> 5) * 1024 + block_at<V>(i & 31, c & 31));
+    };
+    auto U = [&](int i, int c) {
+        return __ldg((const V *)U_ + block_upper(i >> 5, c >> 5) * 1024 + block_at<V>(i & 31, c & 31));
+    };
     bool ovf = false;
 
     // ---------------- forward: unit lower, t = in << bit
@@ -936,15 +980,13 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
         if (k0 > 0) {
             if constexpr (EXACT && VT != VT_I32) {
                 if (tid < kb) {
-                    const V *row = L + (size_t)(k0 + tid) * n;
                     T acc = t[k0 + tid];
-                    for (int c = 0; c < k0; c++) acc = acc_sub<VT, true>(acc, row[c], x[c]);
+                    for (int c = 0; c < k0; c++) acc = acc_sub<VT, true>(acc, L(k0 + tid, c), x[c]);
                     t[k0 + tid] = acc;
                 }
             } else if (warp < kb) {
-                const V *row = L + (size_t)(k0 + warp) * n;
                 T acc = 0;
-                for (int c = lane; c < k0; c += 32) acc = acc_sub<VT, false>(acc, __ldg(row + c), x[c]);
+                for (int c = lane; c < k0; c += 32) acc = acc_sub<VT, false>(acc, L(k0 + warp, c), x[c]);
                 acc = acc_reduce<VT>(acc, 32);
                 if (lane == 0) {
                     if constexpr (VT == VT_I32) t[k0 + warp] = wadd(t[k0 + warp], acc);
@@ -955,9 +997,8 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
         __syncthreads();
         if (warp == 0) {
             V dblk[32];
-            const V *row = L + (size_t)(k0 + lane) * n + k0;
 #pragma unroll
-            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c < lane) ? __ldg(row + c) : V(0);
+            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c < lane) ? L(k0 + lane, k0 + c) : V(0);
             T tr = lane < kb ? t[k0 + lane] : T(0);
 #pragma unroll
             for (int c = 0; c < 32; c++) {
@@ -980,21 +1021,18 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
     // ---------------- backward: D^-1 U, last panel first
     for (int i = tid; i < n; i += kLuThreads) t[i] = acc_init<VT>(x[i], bitU);
     __syncthreads();
-    for (int k1 = n; k1 > 0; k1 -= 32) {
-        const int kb = min(32, k1);
-        const int k0 = k1 - kb;
+    for (int k0 = (npan - 1) * 32; k0 >= 0; k0 -= 32) {
+        const int k1 = min(n, k0 + 32), kb = k1 - k0;
         if (k1 < n) {
             if constexpr (EXACT && VT != VT_I32) {
                 if (tid < kb) {
-                    const V *row = U + (size_t)(k0 + tid) * n;
                     T acc = t[k0 + tid];
-                    for (int c = n - 1; c >= k1; c--) acc = acc_sub<VT, true>(acc, row[c], x[c]);
+                    for (int c = n - 1; c >= k1; c--) acc = acc_sub<VT, true>(acc, U(k0 + tid, c), x[c]);
                     t[k0 + tid] = acc;
                 }
             } else if (warp < kb) {
-                const V *row = U + (size_t)(k0 + warp) * n;
                 T acc = 0;
-                for (int c = k1 + lane; c < n; c += 32) acc = acc_sub<VT, false>(acc, __ldg(row + c), x[c]);
+                for (int c = k1 + lane; c < n; c += 32) acc = acc_sub<VT, false>(acc, U(k0 + warp, c), x[c]);
                 acc = acc_reduce<VT>(acc, 32);
                 if (lane == 0) {
                     if constexpr (VT == VT_I32) t[k0 + warp] = wadd(t[k0 + warp], acc);
@@ -1005,9 +1043,8 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
         __syncthreads();
         if (warp == 0) {
             V dblk[32];
-            const V *row = U + (size_t)(k0 + lane) * n + k0;
 #pragma unroll
-            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c > lane && c < kb) ? __ldg(row + c) : V(0);
+            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c > lane && c < kb) ? U(k0 + lane, k0 + c) : V(0);
             T tr = lane < kb ? t[k0 + lane] : T(0);
             const V dv = lane < kb ? dinv[k0 + lane] : V(0);
 #pragma unroll
@@ -1027,26 +1064,338 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
     if (ovf) atomicOr(flags, ST_OVERFLOW);
 }
 
+// ------------------------------------------------- the chain in one cluster
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of this CTA's shared memory location in CTA `rank`
+__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async_u32(unsigned addr, unsigned v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_u64(unsigned addr, unsigned long long v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(bar)
+                 : "memory");
+}
+template <typename T>
+__device__ __forceinline__ unsigned long long bits_of(T v) {
+    if constexpr (std::is_same<T, double>::value) return (unsigned long long)__double_as_longlong(v);
+    else if constexpr (std::is_same<T, float>::value) return (unsigned long long)__float_as_uint(v);
+    else return (unsigned long long)v;
+}
+template <typename T>
+__device__ __forceinline__ T of_bits(unsigned long long v) {
+    if constexpr (std::is_same<T, double>::value) return __longlong_as_double((long long)v);
+    else if constexpr (std::is_same<T, float>::value) return __uint_as_float((unsigned)v);
+    else return (T)v;
+}
+
+// acc + d * x (integers wrap)
+template <int VT>
+__device__ __forceinline__ acc_t<VT> acc_add(acc_t<VT> a, vt_t<VT> d, vt_t<VT> x) {
+    if constexpr (VT == VT_I32) return wadd(a, (long long)d * (long long)x);
+    else return a + d * x;
+}
+
+struct LuSmem {  // byte offsets
+    int ready, xbar, xs, xf, part, ring, bytes;
+};
+template <int VT>
+__host__ __device__ __forceinline__ LuSmem lu_smem(int npan) {
+    const int es = (int)sizeof(vt_t<VT>);
+    LuSmem s;
+    s.ready = 0;                          // CTA 0: panel k's blocks and sum are there (both directions)
+    s.xbar = s.ready + 2 * npan * 8;      // panel k's values are there
+    s.xs = (s.xbar + 2 * npan * 8 + 127) / 128 * 128;  // the values, panel by panel in the chain's order
+    s.xf = s.xs + npan * 32 * es;         // CTA 0: the forward values
+    s.part = s.xf + npan * 32 * es;       // CTA 0: the sums
+    s.ring = s.part + npan * 32 * 8;      // CTA 0: kLuSlots panels of blocks
+    s.bytes = s.ring + kLuSlots * (1 + kLuNear) * 1024 * es;
+    return s;
+}
+
+template <int VT>
+__global__ void __launch_bounds__(32 * kLuWarps, 1)
+k_lu_chain(int n, const void *__restrict__ L_, const void *__restrict__ U_, const void *__restrict__ dinv_, int bitL,
+           int bitU, int dbitU, const void *__restrict__ in_, void *__restrict__ out_, unsigned *flags) {
+    using V = vt_t<VT>;
+    using T = acc_t<VT>;
+    constexpr int NEAR = kLuNear;
+    constexpr int PER = 16 / (int)sizeof(V), QB = 32 / PER;  // entries of a quad; quads of a block's row
+    constexpr unsigned BB = 1024 * sizeof(V);                // bytes of a block
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int npan = (n + 31) / 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    const LuSmem o = lu_smem<VT>(npan);
+    unsigned long long *ready = (unsigned long long *)(smem_raw + o.ready);
+    unsigned long long *xbar = (unsigned long long *)(smem_raw + o.xbar);
+    V *xs = (V *)(smem_raw + o.xs);
+    __shared__ int s_taken, s_dead;  // panels the chain is done with; a wait ran out
+    const V *L = (const V *)L_, *U = (const V *)U_;
+    if (threadIdx.x == 0) {
+        s_taken = 0;
+        s_dead = 0;
+    }
+    for (int k = threadIdx.x; k < 2 * npan; k += 32 * kLuWarps) {
+        mbar_init(ready + k, 1);
+        mbar_init(xbar + k, 1);
+    }
+    fence_mbar_init();
+    __syncthreads();
+    for (int k = threadIdx.x; k < 2 * npan; k += 32 * kLuWarps) mbar_expect_tx(xbar + k, 32 * sizeof(V));
+    cluster_sync_all();
+
+    auto wait = [&](unsigned long long *bar) {
+        if (mbar_try_wait(bar, 0) || *(volatile int *)&s_dead) return;
+        const unsigned long long t0 = globaltimer_ns();
+        while (!mbar_try_wait(bar, 0))
+            if (*(volatile int *)&s_dead || globaltimer_ns() - t0 > kSpinLimitNs) {
+                *(volatile int *)&s_dead = 1;
+                atomicOr(flags, ST_TIMEOUT);
+                return;
+            }
+    };
+
+    if (rank == 0 && warp == 0) {
+        // ------------------------------------------------------- the chain
+        const V *in = (const V *)in_, *dinv = (const V *)dinv_;
+        V *out = (V *)out_, *xf = (V *)(smem_raw + o.xf);
+        const unsigned long long *part = (const unsigned long long *)(smem_raw + o.part);
+        unsigned xs_at[kLuCtas], bar_at[kLuCtas];
+#pragma unroll
+        for (int r = 0; r < kLuCtas; r++) {
+            xs_at[r] = map_rank(smem_addr(xs), r);
+            bar_at[r] = map_rank(smem_addr(xbar), r);
+        }
+        bool ovf = false;
+        for (int dir = 0; dir < 2; dir++) {
+            const bool fwd = dir == 0;
+            T near[NEAR];  // the products of the panels before with the next ones
+#pragma unroll
+            for (int j = 0; j < NEAR; j++) near[j] = T(0);
+            auto row_of = [&](int k) { return (fwd ? k : npan - 1 - k) * 32 + lane; };
+            auto start = [&](int k) {  // the row's input, and its inverse diagonal
+                const int i = row_of(k);
+                return k < npan && i < n ? (fwd ? in[i] : xf[i]) : V(0);
+            };
+            auto dinv_of = [&](int k) {
+                const int i = row_of(k);
+                return !fwd && k < npan && i < n ? __ldg(dinv + i) : V(0);
+            };
+            V s0 = start(0), dv = dinv_of(0);
+            for (int k = 0; k < npan; k++) {
+                const int i = row_of(k);
+                wait(ready + dir * npan + k);
+                T sum = near[0];
+                if (k > NEAR) {
+                    const T far = of_bits<T>(part[k * 32 + lane]);
+                    if constexpr (VT == VT_I32) sum = wadd(sum, far);
+                    else sum += far;
+                }
+#pragma unroll
+                for (int j = 0; j + 1 < NEAR; j++) near[j] = near[j + 1];
+                near[NEAR - 1] = T(0);
+                T t = acc_init<VT>(s0, fwd ? bitL : bitU);
+                if constexpr (VT == VT_I32) t = wsub(t, sum);
+                else t -= sum;
+                const V d_here = dv;
+                s0 = start(k + 1);
+                dv = dinv_of(k + 1);
+                const uint4 *blk = (const uint4 *)(smem_raw + o.ring + (dir * npan + k) % kLuSlots * (1 + NEAR) * BB) + lane;
+                const int bit = fwd ? bitL : bitU;
+                // integers: u = ~t, so that a step is one multiply-add
+                if constexpr (VT == VT_I32) t = ~t;
+                auto value = [&](bool &bad) {  // x of this lane's row as t stands
+                    if constexpr (VT == VT_I32) {
+                        if (fwd) {
+                            const long long s = ~(t >> bit);
+                            bad = !fits32(s);
+                            return lo32(s);
+                        }
+                        bad = false;
+                        return acc_finish<VT>(~t, d_here, bitU, dbitU, bad);
+                    } else {
+                        bad = false;
+                        return fwd ? t : t * d_here;
+                    }
+                };
+                auto steps = [&](auto forward) {
+                    constexpr bool F = decltype(forward)::value;
+#pragma unroll
+                    for (int g = 0; g < QB; g++) {
+                        const int gq = F ? g : QB - 1 - g;
+                        uint4 q[1 + NEAR];
+#pragma unroll
+                        for (int j = 0; j <= NEAR; j++) q[j] = blk[j * (BB / 16) + gq * 32];
+#pragma unroll
+                        for (int e = 0; e < PER; e++) {
+                            const int ec = F ? e : PER - 1 - e, c = gq * PER + ec;
+                            bool bad;
+                            V xc;
+                            if constexpr (VT == VT_I32 && F) xc = ~(int)__funnelshift_r((unsigned)t, (unsigned)((unsigned long long)t >> 32), bit);
+                            else xc = value(bad);
+                            xc = __shfl_sync(0xffffffffu, xc, c);
+                            auto entry = [&](const uint4 &w) {
+                                if constexpr (VT == VT_F64) return ec == 0 ? __hiloint2double((int)w.y, (int)w.x) : __hiloint2double((int)w.w, (int)w.z);
+                                else {
+                                    const unsigned u = ec == 0 ? w.x : ec == 1 ? w.y : ec == 2 ? w.z : w.w;
+                                    if constexpr (VT == VT_I32) return (int)u;
+                                    else return __uint_as_float(u);
+                                }
+                            };
+                            if constexpr (VT == VT_I32) t = acc_add<VT>(t, entry(q[0]), xc);
+                            else if (F ? lane > c : lane < c) t -= entry(q[0]) * xc;  // (0 * inf is no 0)
+#pragma unroll
+                            for (int j = 0; j < NEAR; j++) near[j] = acc_add<VT>(near[j], entry(q[1 + j]), xc);
+                        }
+                    }
+                };
+                if (fwd) steps(std::true_type());
+                else steps(std::false_type());
+                bool bad;
+                V x = value(bad);
+                if (i >= n) {
+                    x = V(0);
+                    bad = false;
+                }
+                ovf |= bad;
+                // to every CTA of the cluster
+                const unsigned at = (unsigned)((k * 32 + lane) * sizeof(V)), bt = (unsigned)((dir * npan + k) * 8);
+#pragma unroll
+                for (int r = 0; r < kLuCtas; r++) {
+                    if constexpr (sizeof(V) == 8) st_async_u64(xs_at[r] + at, bits_of<V>(x), bar_at[r] + bt);
+                    else st_async_u32(xs_at[r] + at, (unsigned)bits_of<V>(x), bar_at[r] + bt);
+                }
+                if (fwd) xf[i] = x;
+                else if (i < n) out[i] = x;
+                __syncwarp();
+                if (lane == 0) *(volatile int *)&s_taken = dir * npan + k + 1;
+            }
+        }
+        if (ovf) atomicOr(flags, ST_OVERFLOW);
+    } else if (rank == 0 && warp == 1) {
+        // ------------------------------------- the loader of the chain's blocks
+        if (lane == 0) {
+            for (int m = 0; m < 2 * npan; m++) {
+                const int k = m < npan ? m : m - npan, have = min(1 + NEAR, npan - k);
+                const unsigned long long t0 = globaltimer_ns();
+                while (*(volatile int *)&s_taken + kLuSlots <= m) {
+                    if (*(volatile int *)&s_dead) break;
+                    if (globaltimer_ns() - t0 > kSpinLimitNs) {
+                        *(volatile int *)&s_dead = 1;
+                        atomicOr(flags, ST_TIMEOUT);
+                    }
+                }
+                if (*(volatile int *)&s_dead) break;
+                const unsigned bytes = have * BB, sum = k > NEAR ? 32 * 8 : 0;
+                mbar_expect_tx(ready + m, bytes + sum);
+                // column panel k: the diagonal block and the ones after it lie side by side
+                const V *src = m < npan ? L + block_lower(npan, k, k) * 1024 : U + block_upper(npan - 1 - k, npan - 1 - k) * 1024;
+                bulk_g2s(smem_raw + o.ring + m % kLuSlots * (1 + NEAR) * BB, src, bytes, ready + m);
+            }
+        }
+    } else if (rank != 0) {
+        // --------------------- sums of a panel's products with the far columns
+        const int h = ((int)rank - 1) * kLuWarps + warp;
+        const unsigned part0 = map_rank(smem_addr(smem_raw + o.part), 0), ready0 = map_rank(smem_addr(ready), 0);
+        for (int dir = 0; dir < 2; dir++) {
+            // (panel NEAR + 1 is the first with far columns)
+            for (int k = NEAR + 1 + h; k < npan; k += kLuHelpers) {
+                T a = T(0), b = T(0);
+                auto block = [&](int j) {  // block (panel k, column panel j), both in the chain's order
+                    const V *base = dir == 0 ? L + block_lower(npan, k, j) * 1024
+                                             : U + block_upper(npan - 1 - k, npan - 1 - j) * 1024;
+                    return (const uint4 *)base + lane;
+                };
+                uint4 w[QB];
+#pragma unroll
+                for (int g = 0; g < QB; g++) w[g] = __ldg(block(0) + g * 32);
+                for (int j = 0; j < k - NEAR; j++) {
+                    wait(xbar + dir * npan + j);
+                    __syncwarp();
+                    const uint4 *xq = (const uint4 *)(xs + j * 32);
+                    const uint4 *nb = block(min(j + 1, k - NEAR - 1));
+#pragma unroll
+                    for (int g = 0; g < QB; g++) {
+                        const uint4 x = xq[g], v = w[g];
+                        w[g] = __ldg(nb + g * 32);
+                        if constexpr (VT == VT_F64) {
+                            a = acc_add<VT>(a, __hiloint2double((int)v.y, (int)v.x), __hiloint2double((int)x.y, (int)x.x));
+                            b = acc_add<VT>(b, __hiloint2double((int)v.w, (int)v.z), __hiloint2double((int)x.w, (int)x.z));
+                        } else if constexpr (VT == VT_F32) {
+                            a = acc_add<VT>(a, __uint_as_float(v.x), __uint_as_float(x.x));
+                            b = acc_add<VT>(b, __uint_as_float(v.y), __uint_as_float(x.y));
+                            a = acc_add<VT>(a, __uint_as_float(v.z), __uint_as_float(x.z));
+                            b = acc_add<VT>(b, __uint_as_float(v.w), __uint_as_float(x.w));
+                        } else {
+                            a = acc_add<VT>(a, (int)v.x, (int)x.x);
+                            b = acc_add<VT>(b, (int)v.y, (int)x.y);
+                            a = acc_add<VT>(a, (int)v.z, (int)x.z);
+                            b = acc_add<VT>(b, (int)v.w, (int)x.w);
+                        }
+                    }
+                }
+                if constexpr (VT == VT_I32) a = wadd(a, b);
+                else a += b;
+                st_async_u64(part0 + (unsigned)(k * 32 + lane) * 8, bits_of<T>(a), ready0 + (unsigned)(dir * npan + k) * 8);
+            }
+        }
+    }
+    // no CTA leaves while a value may still be on its way into its shared memory
+    // (CTA 0 has waited for the sums)
+    if (warp == kLuWarps - 1) {
+        const unsigned long long t0 = globaltimer_ns();
+        for (int m = lane; m < 2 * npan; m += 32)
+            while (!mbar_try_wait(xbar + m, 0) && globaltimer_ns() - t0 <= kSpinLimitNs) {
+            }
+    }
+    __syncthreads();
+    cluster_sync_all();
+}
+
 void DevDenseLU::release() {
     dfree(L);
     dfree(U);
     dfree(dinv);
-    dfree(tmp);
-    L = U = dinv = tmp = nullptr;
+    L = U = dinv = nullptr;
 }
 
+// the triangles in 32 x 32 blocks (see block_at); dutri rows: D^-1 first, then
+// the strict upper entries
 template <typename V>
-static void densify(int n, const int *Lrptr, const int *Lcind, const V *Lval, const int *Urptr, const int *Ucind,
-                    const V *Uval, std::vector<V> &Ld, std::vector<V> &Ud, std::vector<V> &dinv) {
-    Ld.assign((size_t)n * n, V(0));
-    Ud.assign((size_t)n * n, V(0));
-    dinv.assign(n, V(0));
+static void upload_lu_blocks(DevDenseLU &d, const int *Lrptr, const int *Lcind, const V *Lval, const int *Urptr,
+                             const int *Ucind, const V *Uval) {
+    const int n = d.n, npan = (n + 31) / 32;
+    const size_t size = (size_t)npan * (npan + 1) / 2 * 1024;
+    std::vector<V> Lb(size, V(0)), Ub(size, V(0)), dinv(std::max(n, 1), V(0));
     for (int i = 0; i < n; i++) {
-        for (int j = Lrptr[i]; j < Lrptr[i + 1]; j++) Ld[(size_t)i * n + Lcind[j]] = Lval[j];
-        // dutri rows: D^-1 first, then the strict upper entries
+        for (int j = Lrptr[i]; j < Lrptr[i + 1]; j++) {
+            const int c = Lcind[j];
+            if (c >= i) continue;
+            Lb[block_lower(npan, i >> 5, c >> 5) * 1024 + block_at<V>(i & 31, c & 31)] = Lval[j];
+        }
         if (Urptr[i + 1] > Urptr[i]) dinv[i] = Uval[Urptr[i]];
-        for (int j = Urptr[i] + 1; j < Urptr[i + 1]; j++) Ud[(size_t)i * n + Ucind[j]] = Uval[j];
+        for (int j = Urptr[i] + 1; j < Urptr[i + 1]; j++) {
+            const int c = Ucind[j];
+            if (c <= i) continue;
+            Ub[block_upper(i >> 5, c >> 5) * 1024 + block_at<V>(i & 31, c & 31)] = Uval[j];
+        }
     }
+    if (Lb.empty()) Lb.resize(1024);
+    if (Ub.empty()) Ub.resize(1024);
+    d.L = dupload(Lb);
+    d.U = dupload(Ub);
+    d.dinv = dupload(dinv);
 }
 
 DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval, const int *Urptr,
@@ -1057,28 +1406,36 @@ DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval,
     d.bitL = bitL;
     d.bitU = bitU;
     d.dbitU = dbitU;
-    if (vt == VT_I32) {
-        std::vector<int32_t> Ld, Ud, dv;
-        densify(n, Lrptr, Lcind, (const int32_t *)Lval, Urptr, Ucind, (const int32_t *)Uval, Ld, Ud, dv);
-        d.L = dupload(Ld); d.U = dupload(Ud); d.dinv = dupload(dv);
-    } else if (vt == VT_F64) {
-        std::vector<double> Ld, Ud, dv;
-        densify(n, Lrptr, Lcind, (const double *)Lval, Urptr, Ucind, (const double *)Uval, Ld, Ud, dv);
-        d.L = dupload(Ld); d.U = dupload(Ud); d.dinv = dupload(dv);
-    } else {
-        std::vector<float> Ld, Ud, dv;
-        densify(n, Lrptr, Lcind, (const float *)Lval, Urptr, Ucind, (const float *)Uval, Ld, Ud, dv);
-        d.L = dupload(Ld); d.U = dupload(Ud); d.dinv = dupload(dv);
-    }
+    if (vt == VT_I32) upload_lu_blocks(d, Lrptr, Lcind, (const int32_t *)Lval, Urptr, Ucind, (const int32_t *)Uval);
+    else if (vt == VT_F64) upload_lu_blocks(d, Lrptr, Lcind, (const double *)Lval, Urptr, Ucind, (const double *)Uval);
+    else upload_lu_blocks(d, Lrptr, Lcind, (const float *)Lval, Urptr, Ucind, (const float *)Uval);
     return d;
 }
 
 template <int VT, bool EXACT>
 static void launch_lu(Ctx &c, const DevDenseLU &LU, const void *in, void *out) {
+    c.launches++;
+    const int chain = lu_smem<VT>((LU.n + 31) / 32).bytes;
+    if (!EXACT && (size_t)chain <= kLuChainSmem && (VT != VT_I32 || (LU.bitL >= 0 && LU.bitL < 32))) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kLuCtas);
+        cfg.blockDim = dim3(32 * kLuWarps);
+        cfg.dynamicSmemBytes = chain;
+        cfg.stream = c.stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kLuCtas;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        SAGB_CUDA(cudaLaunchKernelEx(&cfg, k_lu_chain<VT>, LU.n, (const void *)LU.L, (const void *)LU.U, (const void *)LU.dinv,
+                                     LU.bitL, LU.bitU, LU.dbitU, in, out, c.d_flags));
+        return;
+    }
     const size_t smem = (sizeof(acc_t<VT>) + sizeof(vt_t<VT>)) * (size_t)LU.n;
     k_dense_lu<VT, EXACT><<<1, kLuThreads, smem, c.stream>>>(LU.n, LU.L, LU.U, LU.dinv, LU.bitL, LU.bitU,
                                                                 LU.dbitU, in, out, c.d_flags);
-    c.launches++;
 }
 
 template <int VT, bool EXACT>
@@ -1088,6 +1445,7 @@ static void cta_attrs() {
         for (int lines = 1; lines <= 4; lines *= 2)
             SAGB_CUDA(cudaFuncSetAttribute(sweep_kernel<VT, EXACT>(lg, lines), cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     SAGB_CUDA(cudaFuncSetAttribute(k_dense_lu<VT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    if (!EXACT) SAGB_CUDA(cudaFuncSetAttribute(k_lu_chain<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
 }
 
 void init_kernel_attributes() {

@@ -153,13 +153,12 @@ void trsv(Ctx &c, const DevTri &T, const void *in, void *out);
 // the same sweep with its scratch in a static device array (no allocation)
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out);
 
-// Dense coarsest-level LU: strict lower L (unit), strict upper U and D^-1,
-// row-major n x n, solved by one block.
+// Dense coarsest-level LU: strict lower L (unit) and strict upper U as 32 x 32
+// blocks of the triangles (cuda/trsv.cu, block_at), and D^-1.
 struct DevDenseLU {
     int n = 0, vt = VT_I32;
     int bitL = 0, bitU = 0, dbitU = 0;
     void *L = nullptr, *U = nullptr, *dinv = nullptr;
-    void *tmp = nullptr;
     void release();
 };
 DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval, const int *Urptr,
