@@ -20,7 +20,7 @@
 
 #include "../sagb_internal.hpp"
 #include "common.cuh"
-#include "stream.cuh"
+#include "rows.cuh"
 
 namespace sagb {
 
@@ -204,37 +204,12 @@ k_spmv_dot_i32(int n, const int *__restrict__ rptr, const int *__restrict__ cind
     const long long tid = (long long)blockIdx.x * kRedThreads + threadIdx.x;
     const int row = (int)(tid / G), lane = (int)(tid % G);
     long long a = 0;
-    if (row < n) {
-        const int b0 = __ldg(rptr + row), b1 = __ldg(rptr + row + 1);
-        for (int j = b0 + lane; j < b1; j += G) a = wadd(a, (long long)__ldg(val + j) * __ldg(z + __ldg(cind + j)));
-    }
+    if (row < n) a = row_part<G>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, z);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) a = wadd(a, shfl_xor(a, o));
     long long d = 0;
     if (lane == 0 && row < n) {
         const long long s = a >> bit;
-        const int y = lo32(s);
-        if (!fits32(s)) atomicOr(flags, ST_OVERFLOW);
-        w[row] = y;
-        d = (long long)__ldg(v0 + row) * y;
-    }
-    d = block_sum(d, sh);
-    if (threadIdx.x == 0) atomicAdd(acc, (unsigned long long)d);
-}
-
-// the same through the tile-staged stream (short rows)
-__global__ void __launch_bounds__(kStreamThreads)
-k_spmv_dot_stream_i32(int n, const int *__restrict__ rptr, const int *__restrict__ cind, const int *__restrict__ val,
-                      const int *__restrict__ z, int *__restrict__ w, const int *__restrict__ v0, int bit,
-                      unsigned long long *acc, unsigned *flags) {
-    __shared__ long long sh[32];
-    long long a[1] = {0};
-    const int r0 = blockIdx.x * kStreamThreads;
-    stream_rows<1>(r0, min(n, r0 + kStreamThreads), rptr, cind, val, z, a);
-    const int row = r0 + threadIdx.x;
-    long long d = 0;
-    if (row < n) {
-        const long long s = a[0] >> bit;
         const int y = lo32(s);
         if (!fits32(s)) atomicOr(flags, ST_OVERFLOW);
         w[row] = y;
@@ -389,10 +364,7 @@ k_spmv_dot_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind,
     const long long tid = (long long)blockIdx.x * kRedThreads + threadIdx.x;
     const int row = (int)(tid / G), lane = (int)(tid % G);
     T a = 0;
-    if (row < n) {
-        const int b0 = __ldg(rptr + row), b1 = __ldg(rptr + row + 1);
-        for (int j = b0 + lane; j < b1; j += G) a += __ldg(val + j) * __ldg(z + __ldg(cind + j));
-    }
+    if (row < n) a = row_part<G>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, z);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) a += shfl_xor(a, o);
     T d = 0;
@@ -732,18 +704,12 @@ class IntSolver : public SolverBase {
             int *vj = V_ + (size_t)j * N, *zj = Z_ + (size_t)j * N, *w = V_ + (size_t)(j + 1) * N;
             StepInfo inf = step(j, [&] {
                 vcycle(c_, *M_, vj, zj);
-                if (A_->group == 0) {
-                    k_spmv_dot_stream_i32<<<(N + kStreamThreads - 1) / kStreamThreads, kStreamThreads, 0,
-                                            c_.stream>>>(N, A_->rptr, A_->cind, (const int *)A_->val, zj, w, V_,
-                                                         A_->bit, acc_, c_.d_flags);
-                } else {
-                    by_group(A_->group, [&](auto G) {
-                        const long long thr = (long long)N * G.value;
-                        const int blocks = (int)((thr + kRedThreads - 1) / kRedThreads);
-                        k_spmv_dot_i32<G.value><<<blocks, kRedThreads, 0, c_.stream>>>(
-                            N, A_->rptr, A_->cind, (const int *)A_->val, zj, w, V_, A_->bit, acc_, c_.d_flags);
-                    });
-                }
+                by_group(A_->group, [&](auto G) {
+                    const long long thr = (long long)N * G.value;
+                    const int blocks = (int)((thr + kRedThreads - 1) / kRedThreads);
+                    k_spmv_dot_i32<G.value><<<blocks, kRedThreads, 0, c_.stream>>>(
+                        N, A_->rptr, A_->cind, (const int *)A_->val, zj, w, V_, A_->bit, acc_, c_.d_flags);
+                });
                 for (int k = 0; k < j; k++)
                     k_mgs_i32<false><<<gb, kRedThreads, 0, c_.stream>>>(N, k, j, m, bit, V_, w, acc_, H_);
                 k_mgs_i32<true><<<gb, kRedThreads, 0, c_.stream>>>(N, j, j, m, bit, V_, w, acc_, H_);

@@ -1,0 +1,70 @@
+// A lane's part of one CSR row's sum, for kernels that give a row G lanes.
+//
+// Bound by memory latency and, with one lane a row, by the L1 cache (each load
+// of a warp touches as many lines as rows): four entries a lane are in flight,
+// the last one to three in one predicated round, and the kernels stay at 32
+// registers, so that an SM holds all its threads.  Poisson 127^3 (FP64, 2.05 M
+// rows of 7 entries), one lane a row: 39.6 us = 5.4 TB/s; one entry at a time
+// and four lanes a row, 131 us.  Copying the entries of 256 rows into shared
+// memory first was slower: 42 us, with the next 256 rows' copy behind the sums
+// 48 us.  A lane adds its entries in their order.
+#pragma once
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace sagb {
+
+template <bool EXACT>
+__device__ __forceinline__ long long row_add(long long a, int v, int x) {
+    return wadd(a, (long long)v * (long long)x);
+}
+template <bool EXACT>  // multiply and add rounded one by one
+__device__ __forceinline__ double row_add(double a, double v, double x) {
+    return EXACT ? __dadd_rn(a, __dmul_rn(v, x)) : a + v * x;
+}
+template <bool EXACT>
+__device__ __forceinline__ float row_add(float a, float v, float x) {
+    return EXACT ? __fadd_rn(a, __fmul_rn(v, x)) : a + v * x;
+}
+
+// entries a + lane, a + lane + G, ... below b
+template <int G, bool EXACT = false, typename V>
+__device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__restrict__ cind, const V *__restrict__ val,
+                                         const V *__restrict__ x) {
+    std::conditional_t<std::is_same<V, int>::value, long long, V> acc = 0;
+    int j = a + lane;
+    for (; j + 3 * G < b; j += 4 * G) {
+        int c[4];
+        V v[4], xv[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            c[q] = __ldg(cind + j + q * G);
+            v[q] = __ldg(val + j + q * G);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) xv[q] = __ldg(x + c[q]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc = row_add<EXACT>(acc, v[q], xv[q]);
+    }
+    if (j + G < b) {
+        const bool third = j + 2 * G < b;
+        int c[3];
+        V v[3], xv[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            c[q] = q < 2 || third ? __ldg(cind + j + q * G) : 0;
+            v[q] = q < 2 || third ? __ldg(val + j + q * G) : V(0);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) xv[q] = q < 2 || third ? __ldg(x + c[q]) : V(0);
+#pragma unroll
+        for (int q = 0; q < 2; q++) acc = row_add<EXACT>(acc, v[q], xv[q]);
+        if (third) acc = row_add<EXACT>(acc, v[2], xv[2]);
+    } else if (j < b) {
+        acc = row_add<EXACT>(acc, __ldg(val + j), __ldg(x + __ldg(cind + j)));
+    }
+    return acc;
+}
+
+}  // namespace sagb

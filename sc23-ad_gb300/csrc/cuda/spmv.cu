@@ -11,7 +11,7 @@
 
 #include "../sagb_internal.hpp"
 #include "common.cuh"
-#include "stream.cuh"
+#include "rows.cuh"
 
 namespace sagb {
 
@@ -37,9 +37,25 @@ void DevCsr::release() {
     val = nullptr;
 }
 
-// integer matrices with at most this many entries per row on average use the
-// tile-staged stream kernel (group 0)
-constexpr double kStreamMaxAvg = 32.0;
+// Lanes per row of the plain SpMV: a twelfth of the average row, so that a lane
+// has several entries in flight and a warp reads few lines at a time, and more in
+// matrices too small to fill the chip that way (up to about a row's entries:
+// there the longest row counts).  Measured us by lanes, 1 / 2 / 4 / 8 / 16 / 32:
+//   FP64 2.05 M rows of 7:    39.6 / 62 / 79 / 133 / 317 / 747
+//   FP64 250 k rows of 55:    60 / 44 / 41 / 65 / 83 / 110
+//   int 250 k rows of 55:     42 / 28 / 26 / 30 / 39 / 58
+//   int 125 k rows of 81:     42 / 26 / 24 / 19 / 22 / 31
+//   FP64 20.8 k rows of 339:  76 / 37 / 27 / 26 / 26 / 28
+//   FP64 2.5 k rows of 258:   71 / 40 / 24 / 14 / 9.9 / 8.7
+// (before: three quarters of the average row, so 4, 32, -, -, 32, 32 of them)
+static int spmv_group(int n, int64_t nnz) {
+    if (n == 0) return 1;
+    const double avg = (double)nnz / n;
+    int g = 1;
+    while (g < 32 && avg > 12 * 1.414 * g) g *= 2;
+    while (g < 32 && (int64_t)n * g < 131072 && g < 0.75 * avg) g *= 2;
+    return g;
+}
 
 int pick_group(double avg) {
     // lanes per row: about the average row length, within [1, 32]
@@ -58,8 +74,7 @@ DevCsr upload_csr_i32(const CsrI &A) {
     d.rptr = dupload(A.rptr);
     d.cind = A.cind.empty() ? (int *)dmalloc(16) : dupload(A.cind);
     d.val = A.val.empty() ? dmalloc(16) : (void *)dupload(A.val);
-    d.group = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
-    if (A.n && (double)d.nnz / A.n <= kStreamMaxAvg) d.group = 0;  // tile-staged stream
+    d.group = spmv_group(A.n, d.nnz);
     return d;
 }
 
@@ -73,7 +88,7 @@ DevCsr upload_csr_fp(const CsrT<T> &A) {
     d.rptr = dupload(A.rptr);
     d.cind = A.cind.empty() ? (int *)dmalloc(16) : dupload(A.cind);
     d.val = A.val.empty() ? dmalloc(16) : (void *)dupload(A.val);
-    d.group = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
+    d.group = spmv_group(A.n, d.nnz);
     return d;
 }
 template DevCsr upload_csr_fp<double>(const CsrT<double> &);
@@ -88,13 +103,34 @@ DevCsr upload_csr_f64(const CsrD &A) {
     d.rptr = dupload(A.rptr);
     d.cind = dupload(A.cind);
     d.val = dupload(A.val);
-    d.group = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
+    d.group = spmv_group(A.n, d.nnz);
     return d;
 }
 
 // ------------------------------------------------------------------ kernels
 
 constexpr int kSpmvThreads = 256;
+
+// y_row from the row's sum; true: an integer left its range
+template <typename V, int MODE, typename T>
+__device__ __forceinline__ bool spmv_store(T acc, int row, V *__restrict__ y, const V *__restrict__ z, int bit) {
+    if constexpr (std::is_same<V, int>::value) {
+        const long long s = acc >> bit;
+        bool ovf = !fits32(s);
+        long long v = (long long)lo32(s);
+        if (MODE == SPMV_RESID) v = (long long)z[row] - v;
+        if (MODE == SPMV_ADD) v = v + (long long)y[row];
+        ovf |= !fits32(v);
+        y[row] = lo32(v);
+        return ovf;
+    } else {
+        T v = acc;
+        if (MODE == SPMV_RESID) v = z[row] - v;
+        if (MODE == SPMV_ADD) v = v + y[row];
+        y[row] = v;
+        return false;
+    }
+}
 
 template <int G, int MODE>
 __global__ void __launch_bounds__(kSpmvThreads)
@@ -105,32 +141,10 @@ k_spmv_i32(int n, const int *__restrict__ rptr, const int *__restrict__ cind, co
     const int row = (int)(tid / G);
     const int lane = (int)(tid % G);
     long long acc = 0;
-    if (row < n) {
-        const int a = __ldg(rptr + row), b = __ldg(rptr + row + 1);
-        int j = a + lane;
-        // four entries per lane in flight (integer sums wrap: any order gives the same result)
-        for (; j + 3 * G < b; j += 4 * G) {
-            const int c0 = __ldg(cind + j), c1 = __ldg(cind + j + G), c2 = __ldg(cind + j + 2 * G),
-                      c3 = __ldg(cind + j + 3 * G);
-            const long long v0 = __ldg(val + j), v1 = __ldg(val + j + G), v2 = __ldg(val + j + 2 * G),
-                            v3 = __ldg(val + j + 3 * G);
-            const long long x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-            acc = wadd(acc, wadd(wadd(v0 * x0, v1 * x1), wadd(v2 * x2, v3 * x3)));
-        }
-        for (; j < b; j += G) acc = wadd(acc, (long long)__ldg(val + j) * (long long)__ldg(x + __ldg(cind + j)));
-    }
+    if (row < n) acc = row_part<G>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, x);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) acc = wadd(acc, shfl_xor(acc, o));
-    if (lane == 0 && row < n) {
-        const long long s = acc >> bit;
-        bool ovf = !fits32(s);
-        long long v = (long long)lo32(s);
-        if (MODE == SPMV_RESID) v = (long long)z[row] - v;
-        if (MODE == SPMV_ADD) v = v + (long long)y[row];
-        ovf |= !fits32(v);
-        y[row] = lo32(v);
-        if (ovf) atomicOr(flags, ST_OVERFLOW);
-    }
+    if (lane == 0 && row < n && spmv_store<int, MODE>(acc, row, y, z, bit)) atomicOr(flags, ST_OVERFLOW);
 }
 
 template <typename T, int G, int MODE, bool EXACT>
@@ -141,61 +155,10 @@ k_spmv_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, con
     const int row = (int)(tid / G);
     const int lane = (int)(tid % G);
     T acc = 0;
-    if (row < n) {
-        const int a = __ldg(rptr + row), b = __ldg(rptr + row + 1);
-        for (int j = a + lane; j < b; j += G) {
-            const T p = __ldg(val + j), q = __ldg(x + __ldg(cind + j));
-            if constexpr (EXACT) {
-                if constexpr (sizeof(T) == 8) acc = __dadd_rn(acc, __dmul_rn(p, q));
-                else acc = __fadd_rn(acc, __fmul_rn(p, q));
-            } else {
-                acc += p * q;
-            }
-        }
-    }
+    if (row < n) acc = row_part<G, EXACT>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, x);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) acc += shfl_xor(acc, o);
-    if (lane == 0 && row < n) {
-        T v = acc;
-        if (MODE == SPMV_RESID) v = z[row] - v;
-        if (MODE == SPMV_ADD) v = v + y[row];
-        y[row] = v;
-    }
-}
-
-// the same rows through the tile-staged stream (short rows)
-template <int MODE>
-__global__ void __launch_bounds__(kStreamThreads)
-k_spmv_stream_i32(int n, const int *__restrict__ rptr, const int *__restrict__ cind, const int *__restrict__ val,
-                  const int *__restrict__ x, int *__restrict__ y, const int *__restrict__ z, int bit,
-                  unsigned *__restrict__ flags) {
-    long long acc[1] = {0};
-    const int r0 = blockIdx.x * kStreamThreads;
-    stream_rows<1>(r0, min(n, r0 + kStreamThreads), rptr, cind, val, x, acc);
-    const int row = r0 + threadIdx.x;
-    if (row < n) {
-        const long long s = acc[0] >> bit;
-        bool ovf = !fits32(s);
-        long long v = (long long)lo32(s);
-        if (MODE == SPMV_RESID) v = (long long)z[row] - v;
-        if (MODE == SPMV_ADD) v = v + (long long)y[row];
-        ovf |= !fits32(v);
-        y[row] = lo32(v);
-        if (ovf) atomicOr(flags, ST_OVERFLOW);
-    }
-}
-
-static void launch_stream_i32(Ctx &c, const DevCsr &A, const void *x, void *y, int mode, const void *z) {
-    const int blocks = (A.n + kStreamThreads - 1) / kStreamThreads;
-    if (blocks == 0) return;
-    auto args = [&](auto kern) {
-        kern<<<blocks, kStreamThreads, 0, c.stream>>>(A.n, A.rptr, A.cind, (const int *)A.val, (const int *)x,
-                                                        (int *)y, (const int *)z, A.bit, c.d_flags);
-    };
-    if (mode == SPMV_SET) args(k_spmv_stream_i32<SPMV_SET>);
-    else if (mode == SPMV_RESID) args(k_spmv_stream_i32<SPMV_RESID>);
-    else args(k_spmv_stream_i32<SPMV_ADD>);
-    c.launches++;
+    if (lane == 0 && row < n) spmv_store<T, MODE>(acc, row, y, z, 0);
 }
 
 template <int G>
@@ -241,10 +204,10 @@ static void dispatch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mod
     }
 }
 
-void spmv(Ctx &c, const DevCsr &A, const void *x, void *y, int mode, const void *z) {
+void spmv(Ctx &c, const DevCsr &A_, const void *x, void *y, int mode, const void *z) {
+    DevCsr A = A_; if (const char *e = getenv("SAGB_GRP")) A.group = atoi(e);
     if (A.vt == VT_I32) {
         switch (A.group) {
-            case 0: return launch_stream_i32(c, A, x, y, mode, z);
             case 1: return launch_i32<1>(c, A, x, y, mode, z);
             case 2: return launch_i32<2>(c, A, x, y, mode, z);
             case 4: return launch_i32<4>(c, A, x, y, mode, z);
