@@ -332,6 +332,8 @@ class BatchEngine {
 // 3-layer FP32 MLP (nin -> hid -> hid -> nout, ReLU on the hidden layers),
 // trained with a masked MSE loss and Adam.  Inputs are standardised on the
 // device with (x - mu) / sd.  Host pointers or device pointers are accepted.
+struct EpochNet;
+
 struct Mlp {
     int nin, hid, nout;
     float *p = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // params, grads, Adam moments
@@ -340,7 +342,8 @@ struct Mlp {
     int ws_batch = 0;
     float *data = nullptr;  // loaded X, T, M
     int data_n = 0, loaded_n = 0;
-    int *perm_d = nullptr;
+    int *perm_d = nullptr;  // bias corrections, row orders and losses of some epochs
+    size_t train_cap = 0;
     long long t = 0;  // Adam step
     Mlp(int in, int hidden, int out, uint64_t seed);
     ~Mlp();
@@ -367,6 +370,8 @@ struct Mlp {
     void gather(Ctx &c, const int *perm, int off, int B, bool targets);
     void forward_batch(Ctx &c, int B);
     void backward_batch(Ctx &c, int B);
+    void launch_epoch(Ctx &c, const EpochNet &net, const int *perm, int n, int batch, float *loss, const float2 *bc,
+                      float lr, float beta1, float beta2, float eps);
     float *loss_slot();
 };
 
