@@ -29,13 +29,13 @@
 #include "../sagb_internal.hpp"
 #include "common.cuh"
 #include "cycle_graph.cuh"
+#include "lu_chain.cuh"
 
 namespace sagb {
 namespace {
 
 constexpr int kFThreads = 256;
 constexpr int kFTileRows = 2048;
-constexpr int kFLuThreads = 512;
 constexpr int kFPkU = 4;  // entries per lane fetched before the launch wait
 
 // ------------------------------------------------------------ vector access
@@ -317,112 +317,19 @@ struct FLuDesc {
     T *out;
 };
 
-// LU<T>::Solve (lu.hpp:35-38) for every system: ltri forward
+// LU<T>::Solve (lu.hpp:35-38) for every system and right-hand side: ltri forward
 // (x_i = in_i - sum_{j<i} l_ij x_j) then dutri backward
-// (x_i = (t_i - sum_{j>i} u_ij x_j) * dinv_i), one CTA per system, 32-row
-// panels: warps reduce panel rows against the solved part, warp 0 solves the
-// diagonal block from registers.
-template <typename T, int R>
-__global__ void __launch_bounds__(kFLuThreads, 1)
-k_flu(const FLuDesc<T> *__restrict__ desc, const T *__restrict__ Lcat, const T *__restrict__ Ucat,
-      const T *__restrict__ dcat) {
+// (x_i = (t_i - sum_{j>i} u_ij x_j) * dinv_i), one cluster each (lu_chain.cuh).
+template <typename T>
+__global__ void __launch_bounds__(32 * kLuWarps, 1)
+k_flu(const FLuDesc<T> *__restrict__ desc, int R, const T *__restrict__ Lcat, const T *__restrict__ Ucat,
+      const T *__restrict__ dcat, unsigned *flags) {
+    constexpr int VT = sizeof(T) == 8 ? VT_F64 : VT_F32;
     pdl_trigger();
-    pdl_wait();
-    extern __shared__ __align__(16) unsigned char fsm[];
-    const FLuDesc<T> d = desc[blockIdx.x];
-    const int n = d.n;
-    T *t = reinterpret_cast<T *>(fsm);
-    T *x = t + (size_t)n * R;
-    const T *L = Lcat + d.mat_off, *U = Ucat + d.mat_off, *dinv = dcat + d.d_off;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = kFLuThreads / 32;
-    for (int i = tid; i < n * R; i += kFLuThreads) t[i] = d.in[i];
-    __syncthreads();
-    for (int k0 = 0; k0 < n; k0 += 32) {
-        const int kb = min(32, n - k0);
-        for (int pr = warp; k0 > 0 && pr < kb; pr += NW) {
-            const T *row = L + (size_t)(k0 + pr) * n;
-            T acc[R];
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] = 0;
-            for (int c = lane; c < k0; c += 32) {
-                const T v = __ldg(row + c);
-#pragma unroll
-                for (int r = 0; r < R; r++) acc[r] += v * x[c * R + r];
-            }
-            lane_reduce<T, R, 32>(acc);
-            if (lane == 0)
-#pragma unroll
-                for (int r = 0; r < R; r++) t[(k0 + pr) * R + r] -= acc[r];
-        }
-        __syncthreads();
-        if (warp == 0) {
-            T blk[32];
-            const T *row = L + (size_t)(k0 + lane) * n + k0;
-#pragma unroll
-            for (int c = 0; c < 32; c++) blk[c] = (lane < kb && c < lane) ? __ldg(row + c) : T(0);
-            T tr[R];
-#pragma unroll
-            for (int r = 0; r < R; r++) tr[r] = lane < kb ? t[(k0 + lane) * R + r] : T(0);
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-                if (c < kb) {
-#pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        const T xc = __shfl_sync(0xffffffffu, tr[r], c);
-                        if (lane > c) tr[r] -= blk[c] * xc;
-                        if (lane == c) x[(k0 + c) * R + r] = xc;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    for (int i = tid; i < n * R; i += kFLuThreads) t[i] = x[i];
-    __syncthreads();
-    for (int k1 = n; k1 > 0; k1 -= 32) {
-        const int kb = min(32, k1);
-        const int k0 = k1 - kb;
-        for (int pr = warp; k1 < n && pr < kb; pr += NW) {
-            const T *row = U + (size_t)(k0 + pr) * n;
-            T acc[R];
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] = 0;
-            for (int c = k1 + lane; c < n; c += 32) {
-                const T v = __ldg(row + c);
-#pragma unroll
-                for (int r = 0; r < R; r++) acc[r] += v * x[c * R + r];
-            }
-            lane_reduce<T, R, 32>(acc);
-            if (lane == 0)
-#pragma unroll
-                for (int r = 0; r < R; r++) t[(k0 + pr) * R + r] -= acc[r];
-        }
-        __syncthreads();
-        if (warp == 0) {
-            T blk[32];
-            const T *row = U + (size_t)(k0 + lane) * n + k0;
-#pragma unroll
-            for (int c = 0; c < 32; c++) blk[c] = (lane < kb && c > lane && c < kb) ? __ldg(row + c) : T(0);
-            T tr[R];
-#pragma unroll
-            for (int r = 0; r < R; r++) tr[r] = lane < kb ? t[(k0 + lane) * R + r] : T(0);
-            const T dv = lane < kb ? __ldg(dinv + k0 + lane) : T(0);
-#pragma unroll
-            for (int c = 31; c >= 0; c--) {
-                if (c < kb) {
-#pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        const T xc = __shfl_sync(0xffffffffu, tr[r] * dv, c);
-                        if (lane < c) tr[r] -= blk[c] * xc;
-                        if (lane == c) x[(k0 + c) * R + r] = xc;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    for (int i = tid; i < n * R; i += kFLuThreads) d.out[i] = x[i];
+    const int id = blockIdx.x / kLuCtas, r = id % R;
+    const FLuDesc<T> d = desc[id / R];
+    const LuChain<VT> a = {d.n, 0, 0, 0, Lcat + d.mat_off, Ucat + d.mat_off, dcat + d.d_off, d.in + r, d.out + r, R};
+    lu_chain<VT, true>(a, flags);
 }
 
 // ============================================================== Krylov
@@ -934,15 +841,22 @@ class FpImpl : public BatchFpEngine::Base {
             d.d_off = (long long)dh.size();
             d.in = ee[lu.level] + (size_t)lu.offset * Rn;
             d.out = xx[lu.level] + (size_t)lu.offset * Rn;
-            Lh.insert(Lh.end(), lu.L.begin(), lu.L.end());
-            Uh.insert(Uh.end(), lu.U.begin(), lu.U.end());
+            LuBlocks<T> B(lu.n);
+            for (int i = 0; i < lu.n; i++) {
+                for (int j = 0; j < i; j++) B.L[B.lower(i, j)] = lu.L[(size_t)i * lu.n + j];
+                for (int j = i + 1; j < lu.n; j++) B.U[B.upper(i, j)] = lu.U[(size_t)i * lu.n + j];
+                B.dinv[i] = lu.dinv[i];
+            }
+            if (sizeof(T) == 8) B.scale_columns();
+            Lh.insert(Lh.end(), B.L.begin(), B.L.end());
+            Uh.insert(Uh.end(), B.U.begin(), B.U.end());
             dh.insert(dh.end(), lu.dinv.begin(), lu.dinv.end());
             maxn = std::max(maxn, (size_t)lu.n);
             desc.push_back(d);
         }
         nlu = (int)desc.size();
-        lu_smem = 2 * sizeof(T) * maxn * Rn;
-        if (lu_smem > 227 * 1024) throw CudaError{"a coarsest level is too large for the batched FP LU kernel"};
+        lu_smem = ::sagb::lu_smem<sizeof(T) == 8 ? VT_F64 : VT_F32>((int)(maxn + 31) / 32).bytes;
+        if (2 * sizeof(T) * maxn * Rn > 227 * 1024) throw CudaError{"a coarsest level is too large for the batched FP LU kernel"};
         Lcat = dupload(Lh);
         Ucat = dupload(Uh);
         dcat = dupload(dh);
@@ -966,9 +880,7 @@ class FpImpl : public BatchFpEngine::Base {
         ascal = (T *)dmalloc(sizeof(T) * (size_t)S * Rn);
         info_d = (FInfo *)dmalloc(sizeof(FInfo));
         SAGB_CUDA(cudaMallocHost(&info_h, sizeof(FInfo)));
-        SAGB_CUDA(cudaFuncSetAttribute(k_flu<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        SAGB_CUDA(cudaFuncSetAttribute(k_flu<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        SAGB_CUDA(cudaFuncSetAttribute(k_flu<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        SAGB_CUDA(cudaFuncSetAttribute(k_flu<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
     }
 
     // LD in colour-row order: items {row, first entry, entries, 0}, the
@@ -1056,16 +968,27 @@ class FpImpl : public BatchFpEngine::Base {
     }
     template <typename... KArgs, typename... Args>
     void launch(void (*k)(KArgs...), int grid, int block, size_t smem, Args... args) {
+        launch_cluster(k, grid, block, smem, 1, args...);
+    }
+    template <typename... KArgs, typename... Args>
+    void launch_cluster(void (*k)(KArgs...), int grid, int block, size_t smem, int cluster, Args... args) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(block);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = c.stream;
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
         int na = 0;
         if (c.use_pdl) {
             at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             at[na].val.programmaticStreamSerializationAllowed = 1;
+            na++;
+        }
+        if (cluster > 1) {
+            at[na].id = cudaLaunchAttributeClusterDimension;
+            at[na].val.clusterDim.x = cluster;
+            at[na].val.clusterDim.y = 1;
+            at[na].val.clusterDim.z = 1;
             na++;
         }
         cfg.attrs = at;
@@ -1125,11 +1048,8 @@ class FpImpl : public BatchFpEngine::Base {
 
     void lu() {
         if (!nlu) return;
-        by_r([&](auto RR) {
-            constexpr int R = decltype(RR)::value;
-            launch(k_flu<T, R>, nlu, kFLuThreads, lu_smem, (const FLuDesc<T> *)d_lu, (const T *)Lcat,
-                   (const T *)Ucat, (const T *)dcat);
-        });
+        launch_cluster(k_flu<T>, kLuCtas * nlu * Rn, 32 * kLuWarps, lu_smem, kLuCtas, (const FLuDesc<T> *)d_lu, Rn,
+                       (const T *)Lcat, (const T *)Ucat, (const T *)dcat, c.d_flags);
     }
 
     // one-colour levels below the finest with their sweeps fused into the

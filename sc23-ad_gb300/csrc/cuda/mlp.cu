@@ -170,9 +170,9 @@ __global__ void k_gather_norm(const float *__restrict__ X, const float *__restri
 // and gradients into all CTAs.  After the first barrier each thread sums the
 // gradient of its own parameter over the batch, updates it (moments in
 // registers) and writes it into all CTAs; the second barrier ends the step.
-// Every sum runs in the order of the kernels above.  A step at 20-64-64-22, with 32
-// / 64 / 100 rows: 11.5 / 13.8 / 17.6 us, 1,109 rows,
-// batches of 64, two epochs: 3,020 -> 590 us with the copies of the data.
+// Every sum runs in the order of the kernels above.  A step at 20-64-64-22 with 32
+// / 64 / 100 rows: 11.5 / 13.8 / 17.6 us; 1,109 rows, batches of 64, two epochs:
+// 3,020 -> 590 us with the copies of the data.
 constexpr int kEpochCtas = 8, kEpochThreads = 1024;
 constexpr int kEpochParams = kEpochCtas * kEpochThreads;  // a parameter a thread
 constexpr int kTrainRows = 1 << 18;                       // rows of the epochs prepared at a time

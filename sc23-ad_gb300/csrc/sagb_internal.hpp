@@ -154,11 +154,11 @@ void trsv(Ctx &c, const DevTri &T, const void *in, void *out);
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out);
 
 // Dense coarsest-level LU: strict lower L (unit) and strict upper U as 32 x 32
-// blocks of the triangles (cuda/trsv.cu, block_at), and D^-1.
+// blocks of the triangles (cuda/lu_chain.cuh), and D^-1; FP64 also U D^-1.
 struct DevDenseLU {
     int n = 0, vt = VT_I32;
     int bitL = 0, bitU = 0, dbitU = 0;
-    void *L = nullptr, *U = nullptr, *dinv = nullptr;
+    void *L = nullptr, *U = nullptr, *W = nullptr, *dinv = nullptr;
     void release();
 };
 DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval, const int *Urptr,
