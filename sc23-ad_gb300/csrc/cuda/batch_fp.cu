@@ -94,12 +94,35 @@ __device__ __forceinline__ void fst(T *x, int row, const T (&v)[R]) {
     }
 }
 
+// The sums of a row's R values over its G lanes, R / min(R, G) of them to a lane:
+// the first exchanges halve the values, the rest are a butterfly.  An FP64 addition keeps a scheduler
+// busy for 64 cycles whatever lanes take part, so the G lanes also share the row's
+// epilogue: at R = 2 and G = 16 a row costs 6 additions and products after its
+// entries instead of 12.
+template <int R, int G>
+struct Share {
+    static constexpr int S = R < G ? R : G;  // lanes that hold sums
+    static constexpr int K = R / S;          // values each
+    static constexpr int L = G / S;          // lanes between them
+};
 template <typename T, int R, int G>
-__device__ __forceinline__ void lane_reduce(T (&a)[R]) {
+__device__ __forceinline__ void lane_share(T (&a)[R], int lane, T (&out)[Share<R, G>::K]) {
+    constexpr int K = Share<R, G>::K;
 #pragma unroll
-    for (int r = 0; r < R; r++)
+    for (int cur = R, o = G / 2; cur > K; cur /= 2, o /= 2) {
+        const bool up = (lane & o) != 0;
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) a[r] += __shfl_xor_sync(0xffffffffu, a[r], o);
+        for (int i = 0; i < cur / 2; i++) {
+            const T keep = up ? a[cur / 2 + i] : a[i], give = up ? a[i] : a[cur / 2 + i];
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+#pragma unroll
+        for (int o = Share<R, G>::L / 2; o > 0; o >>= 1) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
+        out[i] = a[i];
+    }
 }
 
 template <typename T>
@@ -197,35 +220,34 @@ k_fspmv(FMat<T> A, const T *__restrict__ x, T *__restrict__ y, const T *__restri
         for (int r = 0; r < R; r++) acc[r] += vv[q] * xv[r];
     }
     if (e1 - e0 > kPre * G) row_acc<T, R, G, 0>(A.cind, A.val, e0 + lane + kPre * G, e1, x, acc);
-    lane_reduce<T, R, G>(acc);
-    if (lane == 0 && ok) {
-        T out[R];
+    constexpr int K = Share<R, G>::K, L = Share<R, G>::L;
+    T out[K];
+    lane_share<T, R, G>(acc, lane, out);
+    if (lane % L == 0 && ok) {
+        const size_t at = (size_t)row * R + lane / L * K;
         if (mode == SPMV_RESID) {
-            T zz[R];
-            fld<T, R, 0>(z, row, zz);
+            T zz[K];
+            fld<T, K, 0>(z + at, 0, zz);
 #pragma unroll
-            for (int r = 0; r < R; r++) out[r] = zz[r] - acc[r];
+            for (int r = 0; r < K; r++) out[r] = zz[r] - out[r];
         } else if (mode == SPMV_ADD) {
-            T yy[R];
-            fld<T, R, 1>(y, row, yy);
+            T yy[K];
+            fld<T, K, 1>(y + at, 0, yy);
 #pragma unroll
-            for (int r = 0; r < R; r++) out[r] = acc[r] + yy[r];
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; r++) out[r] = acc[r];
+            for (int r = 0; r < K; r++) out[r] = out[r] + yy[r];
         }
         if (jac == 2) {
             const T dinv = __ldg(J.dinv + row);
 #pragma unroll
-            for (int r = 0; r < R; r++) out[r] = (out[r] - T(0)) * dinv;
+            for (int r = 0; r < K; r++) out[r] = (out[r] - T(0)) * dinv;
         }
-        fst<T, R>(y, row, out);
+        fst<T, K>(y + at, 0, out);
         if (jac == 1 && row < J.n) {
             const T dinv = __ldg(J.dinv + row);
-            T x2[R];
+            T x2[K];
 #pragma unroll
-            for (int r = 0; r < R; r++) x2[r] = (out[r] - T(0)) * dinv;
-            fst<T, R>(J.x2, row, x2);
+            for (int r = 0; r < K; r++) x2[r] = (out[r] - T(0)) * dinv;
+            fst<T, K>(J.x2 + at, 0, x2);
         }
     }
 }
@@ -249,14 +271,17 @@ k_fcolour(int cnt, const int *__restrict__ rows, FMat<T> LD, const T *__restrict
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = 0;
     if (k < cnt) row_acc<T, R, G, 1>(LD.cind, LD.val, e0 + lane, dpos, out, acc);
-    lane_reduce<T, R, G>(acc);
-    if (lane == 0 && k < cnt) {
+    constexpr int K = Share<R, G>::K, L = Share<R, G>::L;
+    T res[K];
+    lane_share<T, R, G>(acc, lane, res);
+    if (lane % L == 0 && k < cnt) {
+        const size_t at = (size_t)row * R + lane / L * K;
         const T dinv = __ldg(LD.val + dpos);
-        T iv[R], res[R];
-        fld<T, R, 0>(in, row, iv);
+        T iv[K];
+        fld<T, K, 0>(in + at, 0, iv);
 #pragma unroll
-        for (int r = 0; r < R; r++) res[r] = (iv[r] - acc[r]) * dinv;
-        fst<T, R>(out, row, res);
+        for (int r = 0; r < K; r++) res[r] = (iv[r] - res[r]) * dinv;
+        fst<T, K>(out + at, 0, res);
     }
 }
 
@@ -285,8 +310,10 @@ k_fcolour_packed(int ib, int ie, const int4 *__restrict__ items, const T *__rest
         vv[u] = j < hd.z ? __ldg(eval + hd.y + j) : T(0);
     }
     pdl_wait();
-    T iv[R];
-    if (ok) fld<T, R, 0>(in, hd.x, iv);
+    constexpr int K = Share<R, G>::K, L = Share<R, G>::L;
+    const size_t at = (size_t)hd.x * R + lane / L * K;
+    T iv[K];
+    if (ok && lane % L == 0) fld<T, K, 0>(in + at, 0, iv);
     T acc[R];
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = 0;
@@ -299,12 +326,12 @@ k_fcolour_packed(int ib, int ie, const int4 *__restrict__ items, const T *__rest
         for (int r = 0; r < R; r++) acc[r] += vv[u] * xv[r];
     }
     if (hd.z > kFPkU * G) row_acc<T, R, G, 1>(ecol + hd.y, eval + hd.y, lane + kFPkU * G, hd.z, out, acc);
-    lane_reduce<T, R, G>(acc);
-    if (lane == 0 && ok) {
-        T res[R];
+    T res[K];
+    lane_share<T, R, G>(acc, lane, res);
+    if (lane % L == 0 && ok) {
 #pragma unroll
-        for (int r = 0; r < R; r++) res[r] = (iv[r] - acc[r]) * dinv;
-        fst<T, R>(out, hd.x, res);
+        for (int r = 0; r < K; r++) res[r] = (iv[r] - res[r]) * dinv;
+        fst<T, K>(out + at, 0, res);
     }
 }
 
@@ -319,17 +346,120 @@ struct FLuDesc {
 
 // LU<T>::Solve (lu.hpp:35-38) for every system and right-hand side: ltri forward
 // (x_i = in_i - sum_{j<i} l_ij x_j) then dutri backward
-// (x_i = (t_i - sum_{j>i} u_ij x_j) * dinv_i), one cluster each (lu_chain.cuh).
-template <typename T>
+// (x_i = (t_i - sum_{j>i} u_ij x_j) * dinv_i): FP64 one cluster each (lu_chain.cuh).
 __global__ void __launch_bounds__(32 * kLuWarps, 1)
-k_flu(const FLuDesc<T> *__restrict__ desc, int R, const T *__restrict__ Lcat, const T *__restrict__ Ucat,
-      const T *__restrict__ dcat, unsigned *flags) {
-    constexpr int VT = sizeof(T) == 8 ? VT_F64 : VT_F32;
+k_flu_chain(const FLuDesc<double> *__restrict__ desc, int R, const double *__restrict__ Lcat,
+            const double *__restrict__ Ucat, const double *__restrict__ dcat, unsigned *flags) {
     pdl_trigger();
     const int id = blockIdx.x / kLuCtas, r = id % R;
-    const FLuDesc<T> d = desc[id / R];
-    const LuChain<VT> a = {d.n, 0, 0, 0, Lcat + d.mat_off, Ucat + d.mat_off, dcat + d.d_off, d.in + r, d.out + r, R};
-    lu_chain<VT, true>(a, flags);
+    const FLuDesc<double> d = desc[id / R];
+    const LuChain<VT_F64> a = {d.n, 0, 0, 0, Lcat + d.mat_off, Ucat + d.mat_off, dcat + d.d_off, d.in + r, d.out + r, R};
+    lu_chain<VT_F64, true>(a, flags);
+}
+
+// FP32: one CTA per system, 32-row panels: warps reduce panel rows against the
+// solved part, warp 0 solves the diagonal block from registers.  An FP32 solve's
+// iterations follow the last bits, and the chain's sums have another order.
+constexpr int kFLuThreads = 512;
+template <typename T, int R>
+__global__ void __launch_bounds__(kFLuThreads, 1)
+k_flu_cta(const FLuDesc<T> *__restrict__ desc, const T *__restrict__ Lcat, const T *__restrict__ Ucat,
+      const T *__restrict__ dcat) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) unsigned char fsm[];
+    const FLuDesc<T> d = desc[blockIdx.x];
+    const int n = d.n;
+    T *t = reinterpret_cast<T *>(fsm);
+    T *x = t + (size_t)n * R;
+    const T *L = Lcat + d.mat_off, *U = Ucat + d.mat_off, *dinv = dcat + d.d_off;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NW = kFLuThreads / 32;
+    for (int i = tid; i < n * R; i += kFLuThreads) t[i] = d.in[i];
+    __syncthreads();
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int kb = min(32, n - k0);
+        for (int pr = warp; k0 > 0 && pr < kb; pr += NW) {
+            const T *row = L + (size_t)(k0 + pr) * n;
+            T acc[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) acc[r] = 0;
+            for (int c = lane; c < k0; c += 32) {
+                const T v = __ldg(row + c);
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] += v * x[c * R + r];
+            }
+            T own[1];
+            lane_share<T, R, 32>(acc, lane, own);
+            if (lane % Share<R, 32>::L == 0) t[(k0 + pr) * R + lane / Share<R, 32>::L] -= own[0];
+        }
+        __syncthreads();
+        if (warp == 0) {
+            T blk[32];
+            const T *row = L + (size_t)(k0 + lane) * n + k0;
+#pragma unroll
+            for (int c = 0; c < 32; c++) blk[c] = (lane < kb && c < lane) ? __ldg(row + c) : T(0);
+            T tr[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) tr[r] = lane < kb ? t[(k0 + lane) * R + r] : T(0);
+#pragma unroll
+            for (int c = 0; c < 32; c++) {
+                if (c < kb) {
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const T xc = __shfl_sync(0xffffffffu, tr[r], c);
+                        if (lane > c) tr[r] -= blk[c] * xc;
+                        if (lane == c) x[(k0 + c) * R + r] = xc;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < n * R; i += kFLuThreads) t[i] = x[i];
+    __syncthreads();
+    for (int k1 = n; k1 > 0; k1 -= 32) {
+        const int kb = min(32, k1);
+        const int k0 = k1 - kb;
+        for (int pr = warp; k1 < n && pr < kb; pr += NW) {
+            const T *row = U + (size_t)(k0 + pr) * n;
+            T acc[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) acc[r] = 0;
+            for (int c = k1 + lane; c < n; c += 32) {
+                const T v = __ldg(row + c);
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] += v * x[c * R + r];
+            }
+            T own[1];
+            lane_share<T, R, 32>(acc, lane, own);
+            if (lane % Share<R, 32>::L == 0) t[(k0 + pr) * R + lane / Share<R, 32>::L] -= own[0];
+        }
+        __syncthreads();
+        if (warp == 0) {
+            T blk[32];
+            const T *row = U + (size_t)(k0 + lane) * n + k0;
+#pragma unroll
+            for (int c = 0; c < 32; c++) blk[c] = (lane < kb && c > lane && c < kb) ? __ldg(row + c) : T(0);
+            T tr[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) tr[r] = lane < kb ? t[(k0 + lane) * R + r] : T(0);
+            const T dv = lane < kb ? __ldg(dinv + k0 + lane) : T(0);
+#pragma unroll
+            for (int c = 31; c >= 0; c--) {
+                if (c < kb) {
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const T xc = __shfl_sync(0xffffffffu, tr[r] * dv, c);
+                        if (lane < c) tr[r] -= blk[c] * xc;
+                        if (lane == c) x[(k0 + c) * R + r] = xc;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < n * R; i += kFLuThreads) d.out[i] = x[i];
 }
 
 // ============================================================== Krylov
@@ -353,18 +483,15 @@ struct FInfo {
 template <typename T, int R>
 __device__ __forceinline__ void block_sum_all(T (&v)[R], T (*sh)[R]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    lane_reduce<T, R, 32>(v);
-    if (lane == 0)
-#pragma unroll
-        for (int r = 0; r < R; r++) sh[warp][r] = v[r];
+    T own[1];
+    lane_share<T, R, 32>(v, lane, own);
+    if (lane % Share<R, 32>::L == 0) sh[warp][lane / Share<R, 32>::L] = own[0];
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < R) {  // a value a lane
+        T s = 0;
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            T s = 0;
-            for (int w = 0; w < kFThreads / 32; w++) s += sh[w][r];
-            sh[0][r] = s;
-        }
+        for (int w = 0; w < kFThreads / 32; w++) s += sh[w][threadIdx.x];
+        sh[0][threadIdx.x] = s;
     }
     __syncthreads();
 #pragma unroll
@@ -430,24 +557,30 @@ k_fspmv_dot(const FTile *__restrict__ tiles, FMat<T> A, const T *__restrict__ z,
     __shared__ T sh[kFThreads / 32][R];
     const FTile t = tiles[blockIdx.x];
     const int lane = threadIdx.x % G;
-    T dot[R];
+    constexpr int K = Share<R, G>::K, L = Share<R, G>::L;
+    T mine[K];
 #pragma unroll
-    for (int r = 0; r < R; r++) dot[r] = 0;
+    for (int r = 0; r < K; r++) mine[r] = 0;
     for (int row0 = t.row0; row0 < t.row1; row0 += kFThreads / G) {
         const int row = row0 + threadIdx.x / G;
         T a[R];
 #pragma unroll
         for (int r = 0; r < R; r++) a[r] = 0;
         if (row < t.row1) row_acc<T, R, G, 0>(A.cind, A.val, __ldg(A.rptr + row) + lane, __ldg(A.rptr + row + 1), z, a);
-        lane_reduce<T, R, G>(a);
-        if (lane == 0 && row < t.row1) {
-            T vv[R];
-            fld<T, R, 0>(v0, row, vv);
+        T own[K];
+        lane_share<T, R, G>(a, lane, own);
+        if (lane % L == 0 && row < t.row1) {
+            const size_t at = (size_t)row * R + lane / L * K;
+            T vv[K];
+            fld<T, K, 0>(v0 + at, 0, vv);
 #pragma unroll
-            for (int r = 0; r < R; r++) dot[r] += vv[r] * a[r];
-            fst<T, R>(w, row, a);
+            for (int r = 0; r < K; r++) mine[r] += vv[r] * own[r];
+            fst<T, K>(w + at, 0, own);
         }
     }
+    T dot[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) dot[r] = lane % L == 0 && lane / L == r / K ? mine[r % K] : T(0);
     block_sum_all<T, R>(dot, sh);
     if (threadIdx.x == 0)
 #pragma unroll
@@ -841,22 +974,28 @@ class FpImpl : public BatchFpEngine::Base {
             d.d_off = (long long)dh.size();
             d.in = ee[lu.level] + (size_t)lu.offset * Rn;
             d.out = xx[lu.level] + (size_t)lu.offset * Rn;
-            LuBlocks<T> B(lu.n);
-            for (int i = 0; i < lu.n; i++) {
-                for (int j = 0; j < i; j++) B.L[B.lower(i, j)] = lu.L[(size_t)i * lu.n + j];
-                for (int j = i + 1; j < lu.n; j++) B.U[B.upper(i, j)] = lu.U[(size_t)i * lu.n + j];
-                B.dinv[i] = lu.dinv[i];
+            if constexpr (sizeof(T) == 8) {
+                LuBlocks<T> B(lu.n);
+                for (int i = 0; i < lu.n; i++) {
+                    for (int j = 0; j < i; j++) B.L[B.lower(i, j)] = lu.L[(size_t)i * lu.n + j];
+                    for (int j = i + 1; j < lu.n; j++) B.U[B.upper(i, j)] = lu.U[(size_t)i * lu.n + j];
+                    B.dinv[i] = lu.dinv[i];
+                }
+                B.scale_columns();
+                Lh.insert(Lh.end(), B.L.begin(), B.L.end());
+                Uh.insert(Uh.end(), B.U.begin(), B.U.end());
+            } else {
+                Lh.insert(Lh.end(), lu.L.begin(), lu.L.end());
+                Uh.insert(Uh.end(), lu.U.begin(), lu.U.end());
             }
-            if (sizeof(T) == 8) B.scale_columns();
-            Lh.insert(Lh.end(), B.L.begin(), B.L.end());
-            Uh.insert(Uh.end(), B.U.begin(), B.U.end());
             dh.insert(dh.end(), lu.dinv.begin(), lu.dinv.end());
             maxn = std::max(maxn, (size_t)lu.n);
             desc.push_back(d);
         }
         nlu = (int)desc.size();
-        lu_smem = ::sagb::lu_smem<sizeof(T) == 8 ? VT_F64 : VT_F32>((int)(maxn + 31) / 32).bytes;
-        if (2 * sizeof(T) * maxn * Rn > 227 * 1024) throw CudaError{"a coarsest level is too large for the batched FP LU kernel"};
+        lu_smem = 2 * sizeof(T) * maxn * Rn;
+        if (lu_smem > 227 * 1024) throw CudaError{"a coarsest level is too large for the batched FP LU kernel"};
+        if (sizeof(T) == 8) lu_smem = ::sagb::lu_smem<VT_F64>((int)(maxn + 31) / 32).bytes;
         Lcat = dupload(Lh);
         Ucat = dupload(Uh);
         dcat = dupload(dh);
@@ -880,7 +1019,13 @@ class FpImpl : public BatchFpEngine::Base {
         ascal = (T *)dmalloc(sizeof(T) * (size_t)S * Rn);
         info_d = (FInfo *)dmalloc(sizeof(FInfo));
         SAGB_CUDA(cudaMallocHost(&info_h, sizeof(FInfo)));
-        SAGB_CUDA(cudaFuncSetAttribute(k_flu<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
+        if constexpr (sizeof(T) == 8) {
+            SAGB_CUDA(cudaFuncSetAttribute(k_flu_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
+        } else {
+            SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        }
     }
 
     // LD in colour-row order: items {row, first entry, entries, 0}, the
@@ -1048,8 +1193,15 @@ class FpImpl : public BatchFpEngine::Base {
 
     void lu() {
         if (!nlu) return;
-        launch_cluster(k_flu<T>, kLuCtas * nlu * Rn, 32 * kLuWarps, lu_smem, kLuCtas, (const FLuDesc<T> *)d_lu, Rn,
-                       (const T *)Lcat, (const T *)Ucat, (const T *)dcat, c.d_flags);
+        if constexpr (sizeof(T) == 8)
+            launch_cluster(k_flu_chain, kLuCtas * nlu * Rn, 32 * kLuWarps, lu_smem, kLuCtas, (const FLuDesc<T> *)d_lu, Rn,
+                           (const T *)Lcat, (const T *)Ucat, (const T *)dcat, c.d_flags);
+        else
+            by_r([&](auto RR) {
+                constexpr int R = decltype(RR)::value;
+                launch(k_flu_cta<T, R>, nlu, kFLuThreads, lu_smem, (const FLuDesc<T> *)d_lu, (const T *)Lcat,
+                       (const T *)Ucat, (const T *)dcat);
+            });
     }
 
     // one-colour levels below the finest with their sweeps fused into the
