@@ -822,7 +822,7 @@ class FpSolver : public SolverBase {
                     k_givens_fp<T, true><<<1, 1, 0, c_.stream>>>(j, m, H_, cs_, sn_, e_, sc_, info_d_, c_.d_flags);
                     c_.launches += 2 * j + 4;
                 } else {
-                    by_group(A_->group, [&](auto G) {
+                    by_group(A_->lanes ? A_->lanes : A_->group, [&](auto G) {
                         const long long thr = (long long)N * G.value;
                         const int blocks = (int)((thr + kRedThreads - 1) / kRedThreads);
                         k_spmv_dot_fp<T, G.value><<<blocks, kRedThreads, 0, c_.stream>>>(

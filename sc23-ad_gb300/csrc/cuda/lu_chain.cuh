@@ -1,4 +1,5 @@
-// The dense LU solve of a coarsest level by one thread-block cluster.
+// The dense LU solve of a coarsest level by one thread-block cluster: integers and
+// FP64 (FP32 sums keep an order that the chain does not have).
 #pragma once
 #include <type_traits>
 #include <vector>
@@ -24,18 +25,18 @@ namespace sagb {
 // panel's sum is needed only kLuNear panels after the last value it takes.  Values
 // and sums travel as st.async into the other CTA's shared memory, counted by
 // one mbarrier each; a loader warp brings the chain's blocks ahead of it.
-// Integer sums wrap, so their order does not matter; FP sums are taken in
+// Integer sums wrap, so their order does not matter; FP64 sums are taken in
 // another order than the reference's (the sequential-order mode uses k_dense_lu).
 // Every wait is bounded in time (ST_TIMEOUT); after one that ran out the waits
 // of that CTA no longer wait.
 // FP64: the backward chain runs on t = x / dinv, with the columns of U multiplied
 // by dinv beforehand (one rounding an entry, as the product t dinv has), so that a
 // step of it has one multiply-add and no product.
-// A step is 75-80 cycles for integers and 60 for FP32.  An FP64 multiply-add keeps
-// a scheduler busy for 64: 190 cycles, 155 without the next panel's.  One solve,
+// A step is 75-80 cycles for integers.  An FP64 multiply-add keeps a scheduler
+// busy for 64: 190 cycles, 155 without the next panel's.  One solve,
 // against one CTA with 32-row panels (k_dense_lu on row-major factors): int n = 512
 // 164 -> 43 us, n = 1013 338 -> 82 us, n = 1769 637 -> 142 us; FP64 n = 1013 605 ->
-// 209 us, n = 1872 1,520 -> 381 us; FP32 n = 1013 158 -> 64 us.
+// 209 us, n = 1872 1,520 -> 381 us.
 
 constexpr int kLuCtas = 8;         // k_lu_chain: CTAs of the cluster
 constexpr int kLuWarps = 8;        // and warps of each
@@ -46,13 +47,9 @@ constexpr int kLuSlots = 3;        // panels of the chain's blocks in shared mem
 constexpr int kLuHelpers = (kLuCtas - 1) * kLuWarps;
 // blocks after the diagonal one that the chain takes along: they cover the way of
 // a panel's values to the other CTAs and of a sum back, and cost the chain a
-// multiply-add a step.  1 / 2 / 3 of them: int n = 1769 142 / 146 / 160 us, FP32
-// n = 1013 64 / 64 / 68 us, FP64 n = 1872 521 / 653 us / -
+// multiply-add a step.  1 / 2 / 3 of them: int n = 1769 142 / 146 / 160 us, FP64
+// n = 1872 521 / 653 us / -
 constexpr int kLuNear = 1;
-
-// the backward chain on t = x / dinv
-template <int VT>
-constexpr bool kLuScaled = VT == VT_F64;
 
 // index of element (i, c) of a block triangle: lower (column panel by column
 // panel, downwards from the diagonal) or upper (upwards from the diagonal)
@@ -146,7 +143,7 @@ __host__ __device__ __forceinline__ LuSmem lu_smem(int npan) {
 template <int VT>
 struct LuChain {
     int n, bitL, bitU, dbitU;
-    const vt_t<VT> *L, *U;  // kLuScaled: U's columns times their dinv
+    const vt_t<VT> *L, *U;  // FP64: U's columns times their dinv
     const vt_t<VT> *dinv;
     const vt_t<VT> *in;
     vt_t<VT> *out;
@@ -258,7 +255,7 @@ __device__ __forceinline__ void lu_chain(const LuChain<VT> &a, unsigned *flags) 
                         return acc_finish<VT>(~t, d_here, bitU, dbitU, bad);
                     } else {
                         bad = false;
-                        return fwd || kLuScaled<VT> ? t : t * d_here;
+                        return t;
                     }
                 };
                 auto steps = [&](auto forward) {
@@ -266,7 +263,7 @@ __device__ __forceinline__ void lu_chain(const LuChain<VT> &a, unsigned *flags) 
                     // FP64: the next panel's multiply-adds one group of columns late, or they
                     // come before this panel's in the pipe and hold up the chain
                     constexpr bool kLate = VT == VT_F64;
-                    V le[PER][NEAR], lx[PER];
+                    [[maybe_unused]] V le[PER][NEAR], lx[PER];
                     if constexpr (kLate) {
 #pragma unroll
                         for (int e = 0; e < PER; e++) {
@@ -293,8 +290,7 @@ __device__ __forceinline__ void lu_chain(const LuChain<VT> &a, unsigned *flags) 
                                 if constexpr (VT == VT_F64) return ec == 0 ? __hiloint2double((int)w.y, (int)w.x) : __hiloint2double((int)w.w, (int)w.z);
                                 else {
                                     const unsigned u = ec == 0 ? w.x : ec == 1 ? w.y : ec == 2 ? w.z : w.w;
-                                    if constexpr (VT == VT_I32) return (int)u;
-                                    else return __uint_as_float(u);
+                                    return (int)u;
                                 }
                             };
                             if constexpr (VT == VT_I32) t = acc_add<VT>(t, entry(q[0]), xc);
@@ -336,7 +332,7 @@ __device__ __forceinline__ void lu_chain(const LuChain<VT> &a, unsigned *flags) 
                 }
                 if (i < n) {
                     if constexpr (VT == VT_I32) out[i * ld] = x;
-                    else out[i * ld] = kLuScaled<VT> && !fwd ? x * d_here : x;
+                    else out[i * ld] = fwd ? x : x * d_here;
                 }
                 __syncwarp();
                 if (lane == 0) *(volatile int *)&s_taken = dir * npan + k + 1;
@@ -392,11 +388,6 @@ __device__ __forceinline__ void lu_chain(const LuChain<VT> &a, unsigned *flags) 
                         if constexpr (VT == VT_F64) {
                             sa = acc_add<VT>(sa, __hiloint2double((int)v.y, (int)v.x), __hiloint2double((int)x.y, (int)x.x));
                             sb = acc_add<VT>(sb, __hiloint2double((int)v.w, (int)v.z), __hiloint2double((int)x.w, (int)x.z));
-                        } else if constexpr (VT == VT_F32) {
-                            sa = acc_add<VT>(sa, __uint_as_float(v.x), __uint_as_float(x.x));
-                            sb = acc_add<VT>(sb, __uint_as_float(v.y), __uint_as_float(x.y));
-                            sa = acc_add<VT>(sa, __uint_as_float(v.z), __uint_as_float(x.z));
-                            sb = acc_add<VT>(sb, __uint_as_float(v.w), __uint_as_float(x.w));
                         } else {
                             sa = acc_add<VT>(sa, (int)v.x, (int)x.x);
                             sb = acc_add<VT>(sb, (int)v.y, (int)x.y);

@@ -67,4 +67,34 @@ __device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__re
     return acc;
 }
 
+// The sum that G * V lanes a row give, taken by G: lane g keeps the V partial sums
+// of lanes g, g + G, ..., adds them as their butterfly would, and leaves the rest of
+// the butterfly to the G lanes.  FP32 rows keep their order this way.
+template <int G, int V, typename T>
+__device__ __forceinline__ T row_part_of(int a, int b, int lane, const int *__restrict__ cind, const T *__restrict__ val,
+                                         const T *__restrict__ x) {
+    T acc[V];
+#pragma unroll
+    for (int v = 0; v < V; v++) acc[v] = 0;
+    for (int base = a + lane; base < b; base += G * V) {
+        int c[V];
+        T p[V], q[V];
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            c[v] = base + v * G < b ? __ldg(cind + base + v * G) : -1;
+            p[v] = base + v * G < b ? __ldg(val + base + v * G) : T(0);
+        }
+#pragma unroll
+        for (int v = 0; v < V; v++) q[v] = c[v] >= 0 ? __ldg(x + c[v]) : T(0);
+#pragma unroll
+        for (int v = 0; v < V; v++)
+            if (c[v] >= 0) acc[v] += p[v] * q[v];
+    }
+#pragma unroll
+    for (int o = V / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < o; v++) acc[v] += acc[v + o];
+    return acc[0];
+}
+
 }  // namespace sagb

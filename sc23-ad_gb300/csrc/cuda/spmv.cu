@@ -89,6 +89,10 @@ DevCsr upload_csr_fp(const CsrT<T> &A) {
     d.cind = A.cind.empty() ? (int *)dmalloc(16) : dupload(A.cind);
     d.val = A.val.empty() ? dmalloc(16) : (void *)dupload(A.val);
     d.group = spmv_group(A.n, d.nnz);
+    if (d.vt == VT_F32) {  // the row's sum as by d.lanes lanes (see row_part_of)
+        d.lanes = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
+        d.group = std::min(std::max(d.group, d.lanes / 8), d.lanes);
+    }
     return d;
 }
 template DevCsr upload_csr_fp<double>(const CsrT<double> &);
@@ -147,7 +151,7 @@ k_spmv_i32(int n, const int *__restrict__ rptr, const int *__restrict__ cind, co
     if (lane == 0 && row < n && spmv_store<int, MODE>(acc, row, y, z, bit)) atomicOr(flags, ST_OVERFLOW);
 }
 
-template <typename T, int G, int MODE, bool EXACT>
+template <typename T, int G, int V, int MODE, bool EXACT>  // V: see row_part_of
 __global__ void __launch_bounds__(kSpmvThreads)
 k_spmv_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, const T *__restrict__ val,
           const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ z) {
@@ -155,7 +159,11 @@ k_spmv_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, con
     const int row = (int)(tid / G);
     const int lane = (int)(tid % G);
     T acc = 0;
-    if (row < n) acc = row_part<G, EXACT>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, x);
+    if (row < n) {
+        const int a = __ldg(rptr + row), b = __ldg(rptr + row + 1);
+        if constexpr (V > 1) acc = row_part_of<G, V>(a, b, lane, cind, val, x);
+        else acc = row_part<G, EXACT>(a, b, lane, cind, val, x);
+    }
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) acc += shfl_xor(acc, o);
     if (lane == 0 && row < n) spmv_store<T, MODE>(acc, row, y, z, 0);
@@ -176,7 +184,7 @@ static void launch_i32(Ctx &c, const DevCsr &A, const void *x, void *y, int mode
     c.launches++;
 }
 
-template <typename T, int G, bool EXACT>
+template <typename T, int G, bool EXACT, int V = 1>
 static void launch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mode, const void *z) {
     const long long threads = (long long)A.n * G;
     const int blocks = (int)((threads + kSpmvThreads - 1) / kSpmvThreads);
@@ -185,22 +193,33 @@ static void launch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mode,
         kern<<<blocks, kSpmvThreads, 0, c.stream>>>(A.n, A.rptr, A.cind, (const T *)A.val, (const T *)x, (T *)y,
                                                       (const T *)z);
     };
-    if (mode == SPMV_SET) args(k_spmv_fp<T, G, SPMV_SET, EXACT>);
-    else if (mode == SPMV_RESID) args(k_spmv_fp<T, G, SPMV_RESID, EXACT>);
-    else args(k_spmv_fp<T, G, SPMV_ADD, EXACT>);
+    if (mode == SPMV_SET) args(k_spmv_fp<T, G, V, SPMV_SET, EXACT>);
+    else if (mode == SPMV_RESID) args(k_spmv_fp<T, G, V, SPMV_RESID, EXACT>);
+    else args(k_spmv_fp<T, G, V, SPMV_ADD, EXACT>);
     c.launches++;
 }
 
 template <typename T>
 static void dispatch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mode, const void *z) {
     if (c.fp_exact) return launch_fp<T, 1, true>(c, A, x, y, mode, z);
+    auto by_v = [&](auto G) {
+        constexpr int g = decltype(G)::value;
+        if constexpr (std::is_same<T, float>::value && g <= 16) {
+            if (A.lanes == 2 * g) return launch_fp<T, g, false, 2>(c, A, x, y, mode, z);
+            if constexpr (g <= 8)
+                if (A.lanes == 4 * g) return launch_fp<T, g, false, 4>(c, A, x, y, mode, z);
+            if constexpr (g <= 4)
+                if (A.lanes == 8 * g) return launch_fp<T, g, false, 8>(c, A, x, y, mode, z);
+        }
+        launch_fp<T, g, false>(c, A, x, y, mode, z);
+    };
     switch (A.group) {
-        case 1: return launch_fp<T, 1, false>(c, A, x, y, mode, z);
-        case 2: return launch_fp<T, 2, false>(c, A, x, y, mode, z);
-        case 4: return launch_fp<T, 4, false>(c, A, x, y, mode, z);
-        case 8: return launch_fp<T, 8, false>(c, A, x, y, mode, z);
-        case 16: return launch_fp<T, 16, false>(c, A, x, y, mode, z);
-        default: return launch_fp<T, 32, false>(c, A, x, y, mode, z);
+        case 1: return by_v(std::integral_constant<int, 1>());
+        case 2: return by_v(std::integral_constant<int, 2>());
+        case 4: return by_v(std::integral_constant<int, 4>());
+        case 8: return by_v(std::integral_constant<int, 8>());
+        case 16: return by_v(std::integral_constant<int, 16>());
+        default: return by_v(std::integral_constant<int, 32>());
     }
 }
 

@@ -365,7 +365,8 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 
 constexpr int kSweepThreads = 32 * (kSweepMaxWarps + kSweepImporters);
 
-template <int VT, bool EXACT, int LG, int E>
+// N: lanes that one stands for, each with a sum of its own (FP32, see fixed_lanes)
+template <int VT, bool EXACT, int LG, int E, int N = 1>
 __global__ void __launch_bounds__(kSweepThreads, 1)
 k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
     using V = vt_t<VT>;
@@ -468,7 +469,7 @@ k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
     const unsigned sl = smem_addr(slots);
     int step = 0, need = 0;  // barriers passed, import groups needed
     bool ovf = false, fresh = true;
-    acc_t<VT> t = 0;
+    acc_t<VT> t = 0, tn[N] = {};
     unsigned to = (kSweepStage - 1) * RB, from = RB;  // where the next copy goes and the next record is
     // one record, in registers in r; the next one is brought into n
     auto record = [&](const uint4(&r)[Q], uint4(&n)[Q], bool odd) {
@@ -519,22 +520,40 @@ k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
         for (int q = 0; q < Q; q++) n[q] = lds_quad(mine + from + q * 512);
         from = from == (kSweepStage - 1) * RB ? 0 : from + RB;
         const bool more = c & (1u << 16);  // the row goes on
-        acc_t<VT> s = t, s2 = 0;  // (two chains where the order is free)
-        if constexpr (VT != VT_I32 && LG == 0) s = fresh ? own : t;  // one lane a row: its sum in its order
+        acc_t<VT> s;
+        if constexpr (VT == VT_F32) {  // the lanes' sums in their order; the first starts from the input
+            acc_t<VT> sn[N];
 #pragma unroll
-        for (int h = 0; h < 2 * E; h++) {
-            const uint4 &v = r[1 + h / 2];
-            acc_t<VT> &sum = h < E || EXACT ? s : s2;
-            if constexpr (VT == VT_I32)  // the products, subtracted at the end
-                sum = wadd(sum, (long long)(int)(h & 1 ? v.w : v.y) * (long long)x[h]);
-            else if constexpr (VT == VT_F64)
-                sum = acc_sub<VT, EXACT>(sum, h & 1 ? __hiloint2double((int)v.w, (int)v.z) : __hiloint2double((int)v.y, (int)v.x), x[h]);
-            else
-                sum = acc_sub<VT, EXACT>(sum, __uint_as_float(h & 1 ? v.w : v.y), x[h]);
+            for (int k = 0; k < N; k++) sn[k] = k > 0 ? tn[k] : !fresh ? tn[0] : (lane & ((1 << LG) - 1)) == 0 ? own : V(0);
+#pragma unroll
+            for (int h = 0; h < 2 * E; h++) {
+                const uint4 &v = r[1 + h / 2];
+                sn[h % N] = acc_sub<VT, EXACT>(sn[h % N], __uint_as_float(h & 1 ? v.w : v.y), x[h]);
+            }
+#pragma unroll
+            for (int k = 0; k < N; k++) tn[k] = more ? sn[k] : V(0);
+#pragma unroll
+            for (int o = N / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < o; k++) sn[k] += sn[k + o];
+            s = sn[0];
+        } else {
+            s = t;
+            acc_t<VT> s2 = 0;  // (two chains where the order is free)
+            if constexpr (VT == VT_F64 && LG == 0) s = fresh ? own : t;  // one lane a row: its sum in its order
+#pragma unroll
+            for (int h = 0; h < 2 * E; h++) {
+                const uint4 &v = r[1 + h / 2];
+                acc_t<VT> &sum = h < E || EXACT ? s : s2;
+                if constexpr (VT == VT_I32)  // the products, subtracted at the end
+                    sum = wadd(sum, (long long)(int)(h & 1 ? v.w : v.y) * (long long)x[h]);
+                else
+                    sum = acc_sub<VT, EXACT>(sum, h & 1 ? __hiloint2double((int)v.w, (int)v.z) : __hiloint2double((int)v.y, (int)v.x), x[h]);
+            }
+            if constexpr (VT == VT_I32) s = wadd(s, s2);
+            else if constexpr (!EXACT) s += s2;
+            t = more ? s : acc_t<VT>(0);
         }
-        if constexpr (VT == VT_I32) s = wadd(s, s2);
-        else if constexpr (!EXACT) s += s2;
-        t = more ? s : acc_t<VT>(0);
         fresh = !more;
         s = sweep_sum<VT, LG>(s);
         V dinv;
@@ -542,7 +561,7 @@ k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
         else if constexpr (VT == VT_I32) dinv = (int)r[0].z;
         else dinv = __uint_as_float(r[0].z);
         if constexpr (VT == VT_I32) s = wsub(wshl((long long)own, a.bit), s);
-        else if constexpr (LG > 0) s += own;
+        else if constexpr (LG > 0 && VT == VT_F64) s += own;
         // every lane of a row has its result and stores it
         const V v = acc_finish<VT>(s, dinv, a.bit, a.dbit, ovf);
         sts_unless<V>(c & (1u << 16), row, v);
@@ -615,12 +634,28 @@ static int pow2_at_least(double x) {
     return g;
 }
 
+// Lanes a row where its sum has one order: one in the sequential-order mode.  FP32
+// solves converge in a number of iterations that follows the last bits of their
+// V-cycles, so an FP32 row is summed by both kernels by a number of lanes that
+// depends on its triangle alone: lane g takes entries g, g + G, ... in their order,
+// lane 0 starts from the input, and the lanes are added by a butterfly.  k_sweep may
+// let a lane stand for up to eight of them.  (Lanes and order free, and the coarsest
+// solve on the cluster: an FP32 V-cycle of a 383^2 grid with 40 blocks 714 us
+// instead of 910; but solves of 27-point and variable-coefficient systems took
+// another number of iterations or ended 1e-8 apart.)
+static int fixed_lanes(const Ctx &c, int vt, int n, int64_t off) {
+    if (vt == VT_I32) return 0;
+    if (c.fp_exact) return 1;
+    if (vt == VT_F64) return 0;
+    return pow2_at_least((n ? (double)off / n : 0.0) / ((size_t)n * 4 <= 150 * 1024 ? 4 : kBatch));
+}
+
 static SweepPlan plan_tri(const Ctx &c, const TriSource &t, int vt) {
     SweepLimits lim;
     lim.sms = c.num_sms;
     lim.smem = (int)kSmemMax;
     lim.integer = vt == VT_I32;
-    lim.one_lane = vt != VT_I32 && c.fp_exact;  // sequential order inside a row
+    if (const int g = fixed_lanes(c, vt, t.n, t.n ? (int64_t)t.rptr[t.n] - t.n : 0)) lim.lanes_log = __builtin_ctz(g);
     return build_sweep_plan(t.rptr, t.cind, t.vals, (int)vt_size(vt), t.n, lim, t.level_hint);
 }
 
@@ -642,6 +677,7 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
         d.importers = p.importers;
         d.lg = p.lg;
         d.lines = p.lines;
+        d.virt = p.virt;
         // the small arrays in one buffer (blocks, streams, imports, groups), the
         // records in another
         std::vector<SweepBlock> bl(p.blocks);
@@ -675,7 +711,7 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
         return d;
     }
     const double avg = n ? (double)d.nnz_off / n : 0.0;
-    const int G = vt != VT_I32 && c.fp_exact ? 1 : pow2_at_least(avg / kBatch);  // (sequential order inside a row)
+    const int fixed = fixed_lanes(c, vt, n, d.nnz_off), G = fixed ? fixed : pow2_at_least(avg / kBatch);
     d.group = G;
     const int rows_per_chunk = 2 * kTriThreads / G;
     TriSchedule s = build_tri_schedule(rptr, cind, n, TRI_LD, rows_per_chunk, 1 << 20, src.level_hint);
@@ -752,18 +788,26 @@ static void launch_tri(Ctx &c, const DevTri &T, const void *in, void *out) {
 
 using SweepKernel = void (*)(SweepArgs, const void *, void *, unsigned *);
 template <int VT, bool EXACT, int LG>
-static SweepKernel sweep_kernel_of(int lines) {
+static SweepKernel sweep_kernel_of(int lines, int virt) {
+    if constexpr (VT == VT_F32) {  // (eight entries a record)
+        if constexpr (LG <= 4)
+            if (virt == 1) return k_sweep<VT, EXACT, LG, 4, 2>;
+        if constexpr (LG <= 3)
+            if (virt == 2) return k_sweep<VT, EXACT, LG, 4, 4>;
+        if constexpr (LG <= 2)
+            if (virt == 3) return k_sweep<VT, EXACT, LG, 4, 8>;
+    }
     return lines == 1 ? k_sweep<VT, EXACT, LG, 1> : lines == 2 ? k_sweep<VT, EXACT, LG, 2> : k_sweep<VT, EXACT, LG, 4>;
 }
 template <int VT, bool EXACT>
-static SweepKernel sweep_kernel(int lg, int lines) {
+static SweepKernel sweep_kernel(int lg, int lines, int virt) {
     switch (lg) {
-        case 0: return sweep_kernel_of<VT, EXACT, 0>(lines);
-        case 1: return sweep_kernel_of<VT, EXACT, 1>(lines);
-        case 2: return sweep_kernel_of<VT, EXACT, 2>(lines);
-        case 3: return sweep_kernel_of<VT, EXACT, 3>(lines);
-        case 4: return sweep_kernel_of<VT, EXACT, 4>(lines);
-        default: return sweep_kernel_of<VT, EXACT, 5>(lines);
+        case 0: return sweep_kernel_of<VT, EXACT, 0>(lines, virt);
+        case 1: return sweep_kernel_of<VT, EXACT, 1>(lines, virt);
+        case 2: return sweep_kernel_of<VT, EXACT, 2>(lines, virt);
+        case 3: return sweep_kernel_of<VT, EXACT, 3>(lines, virt);
+        case 4: return sweep_kernel_of<VT, EXACT, 4>(lines, virt);
+        default: return sweep_kernel_of<VT, EXACT, 5>(lines, virt);
     }
 }
 
@@ -774,7 +818,7 @@ static void tri_by_group(Ctx &c, const DevTri &T, const void *in, void *out) {
         while (2 << ilog <= T.importers) ilog++;
         SweepArgs a{T.warps, ilog, T.bit, T.dbit, (const SweepBlock *)T.blocks, T.stream, (const uint4 *)T.data, T.imp_place,
                     T.grp, T.pk, T.sync};
-        sweep_kernel<VT, EXACT>(T.lg, T.lines)<<<T.grid, 32 * (T.warps + T.importers), T.smem,
+        sweep_kernel<VT, EXACT>(T.lg, T.lines, T.virt)<<<T.grid, 32 * (T.warps + T.importers), T.smem,
                                                  c.stream>>>(a, in, out, c.d_flags);
         c.launches++;
         return;
@@ -861,11 +905,12 @@ void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
 // ======================================================== dense coarse LU
 //
 // LUflex::Solve / LU<T>::Solve (solver/lu.hpp:91-94, 30-33) by k_lu_chain (see
-// lu_chain.cuh).  k_dense_lu, one CTA and 32-row panels, left looking, is the
-// sequential-order mode: warps reduce a panel's rows against the solved part (one
-// thread a row in column order where the order counts), then a warp solves the
-// diagonal block; it also takes what the chain does not: fixed-point shifts
-// outside 0..31.
+// lu_chain.cuh).  k_dense_lu, one CTA and 32-row panels, left looking, solves FP32
+// (whose sums keep their order, see fixed_lanes; the chain took 64 us instead of 158
+// at n = 1013), the sequential-order mode and fixed-point shifts outside 0..31:
+// warps reduce a panel's rows against the solved part, lanes over the columns (one
+// thread a row in column order in the sequential-order mode), then a warp solves
+// the diagonal block.  Its factors are stored row by row.
 constexpr int kLuThreads = 1024;
 
 template <int VT, bool EXACT>
@@ -877,16 +922,12 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T *t = (T *)smem_raw;                           // n accumulators
     V *x = (V *)(smem_raw + sizeof(T) * (size_t)n); // n solved values
+    const V *L = (const V *)L_;
+    const V *U = (const V *)U_;
     const V *dinv = (const V *)dinv_;
     const V *in = (const V *)in_;
     V *out = (V *)out_;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, npan = (n + 31) / 32;
-    auto L = [&](int i, int c) {
-        return __ldg((const V *)L_ + block_lower(npan, i >> 5, c >> 5) * 1024 + block_at<V>(i & 31, c & 31));
-    };
-    auto U = [&](int i, int c) {
-        return __ldg((const V *)U_ + block_upper(i >> 5, c >> 5) * 1024 + block_at<V>(i & 31, c & 31));
-    };
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     bool ovf = false;
 
     // ---------------- forward: unit lower, t = in << bit
@@ -898,13 +939,15 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
         if (k0 > 0) {
             if constexpr (EXACT && VT != VT_I32) {
                 if (tid < kb) {
+                    const V *row = L + (size_t)(k0 + tid) * n;
                     T acc = t[k0 + tid];
-                    for (int c = 0; c < k0; c++) acc = acc_sub<VT, true>(acc, L(k0 + tid, c), x[c]);
+                    for (int c = 0; c < k0; c++) acc = acc_sub<VT, true>(acc, row[c], x[c]);
                     t[k0 + tid] = acc;
                 }
             } else if (warp < kb) {
+                const V *row = L + (size_t)(k0 + warp) * n;
                 T acc = 0;
-                for (int c = lane; c < k0; c += 32) acc = acc_sub<VT, false>(acc, L(k0 + warp, c), x[c]);
+                for (int c = lane; c < k0; c += 32) acc = acc_sub<VT, false>(acc, __ldg(row + c), x[c]);
                 acc = acc_reduce<VT>(acc, 32);
                 if (lane == 0) {
                     if constexpr (VT == VT_I32) t[k0 + warp] = wadd(t[k0 + warp], acc);
@@ -915,8 +958,9 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
         __syncthreads();
         if (warp == 0) {
             V dblk[32];
+            const V *row = L + (size_t)(k0 + lane) * n + k0;
 #pragma unroll
-            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c < lane) ? L(k0 + lane, k0 + c) : V(0);
+            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c < lane) ? __ldg(row + c) : V(0);
             T tr = lane < kb ? t[k0 + lane] : T(0);
 #pragma unroll
             for (int c = 0; c < 32; c++) {
@@ -939,18 +983,21 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
     // ---------------- backward: D^-1 U, last panel first
     for (int i = tid; i < n; i += kLuThreads) t[i] = acc_init<VT>(x[i], bitU);
     __syncthreads();
-    for (int k0 = (npan - 1) * 32; k0 >= 0; k0 -= 32) {
-        const int k1 = min(n, k0 + 32), kb = k1 - k0;
+    for (int k1 = n; k1 > 0; k1 -= 32) {
+        const int kb = min(32, k1);
+        const int k0 = k1 - kb;
         if (k1 < n) {
             if constexpr (EXACT && VT != VT_I32) {
                 if (tid < kb) {
+                    const V *row = U + (size_t)(k0 + tid) * n;
                     T acc = t[k0 + tid];
-                    for (int c = n - 1; c >= k1; c--) acc = acc_sub<VT, true>(acc, U(k0 + tid, c), x[c]);
+                    for (int c = n - 1; c >= k1; c--) acc = acc_sub<VT, true>(acc, row[c], x[c]);
                     t[k0 + tid] = acc;
                 }
             } else if (warp < kb) {
+                const V *row = U + (size_t)(k0 + warp) * n;
                 T acc = 0;
-                for (int c = k1 + lane; c < n; c += 32) acc = acc_sub<VT, false>(acc, U(k0 + warp, c), x[c]);
+                for (int c = k1 + lane; c < n; c += 32) acc = acc_sub<VT, false>(acc, __ldg(row + c), x[c]);
                 acc = acc_reduce<VT>(acc, 32);
                 if (lane == 0) {
                     if constexpr (VT == VT_I32) t[k0 + warp] = wadd(t[k0 + warp], acc);
@@ -961,8 +1008,9 @@ k_dense_lu(int n, const void *__restrict__ L_, const void *__restrict__ U_, cons
         __syncthreads();
         if (warp == 0) {
             V dblk[32];
+            const V *row = U + (size_t)(k0 + lane) * n + k0;
 #pragma unroll
-            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c > lane && c < kb) ? U(k0 + lane, k0 + c) : V(0);
+            for (int c = 0; c < 32; c++) dblk[c] = (lane < kb && c > lane && c < kb) ? __ldg(row + c) : V(0);
             T tr = lane < kb ? t[k0 + lane] : T(0);
             const V dv = lane < kb ? dinv[k0 + lane] : V(0);
 #pragma unroll
@@ -990,31 +1038,44 @@ __global__ void __launch_bounds__(32 * kLuWarps, 1) k_lu_chain(LuChain<VT> a, un
 void DevDenseLU::release() {
     dfree(L);
     dfree(U);
-    dfree(W);
+    dfree(Lb);
+    dfree(Ub);
     dfree(dinv);
-    L = U = W = dinv = nullptr;
+    L = U = Lb = Ub = dinv = nullptr;
 }
 
+static bool chain_takes(int vt, int bitL) { return vt == VT_F64 || (vt == VT_I32 && bitL >= 0 && bitL < 32); }
+
 template <typename V>
-static void upload_lu_blocks(DevDenseLU &d, const int *Lrptr, const int *Lcind, const V *Lval, const int *Urptr,
-                             const int *Ucind, const V *Uval) {
+static void upload_lu(DevDenseLU &d, const int *Lrptr, const int *Lcind, const V *Lval, const int *Urptr,
+                      const int *Ucind, const V *Uval) {
     const int n = d.n;
-    LuBlocks<V> B(n);
-    for (int i = 0; i < n; i++) {
-        for (int j = Lrptr[i]; j < Lrptr[i + 1]; j++)
-            if (Lcind[j] < i) B.L[B.lower(i, Lcind[j])] = Lval[j];
-        // dutri rows: D^-1 first, then the strict upper entries
-        if (Urptr[i + 1] > Urptr[i]) B.dinv[i] = Uval[Urptr[i]];
-        for (int j = Urptr[i] + 1; j < Urptr[i + 1]; j++)
-            if (Ucind[j] > i) B.U[B.upper(i, Ucind[j])] = Uval[j];
+    std::vector<V> dinv(std::max(n, 1), V(0));
+    for (int i = 0; i < n; i++)  // dutri rows: D^-1 first, then the strict upper entries
+        if (Urptr[i + 1] > Urptr[i]) dinv[i] = Uval[Urptr[i]];
+    if (chain_takes(d.vt, d.bitL)) {
+        LuBlocks<V> B(n);
+        B.dinv = dinv;
+        for (int i = 0; i < n; i++) {
+            for (int j = Lrptr[i]; j < Lrptr[i + 1]; j++)
+                if (Lcind[j] < i) B.L[B.lower(i, Lcind[j])] = Lval[j];
+            for (int j = Urptr[i] + 1; j < Urptr[i + 1]; j++)
+                if (Ucind[j] > i) B.U[B.upper(i, Ucind[j])] = Uval[j];
+        }
+        if (d.vt == VT_F64) B.scale_columns();
+        d.Lb = dupload(B.L);
+        d.Ub = dupload(B.U);
     }
-    d.L = dupload(B.L);
-    d.U = dupload(B.U);
-    d.dinv = dupload(B.dinv);
-    if (std::is_same<V, double>::value) {
-        B.scale_columns();
-        d.W = dupload(B.U);
+    if (d.vt != VT_I32 || !d.Lb) {
+        std::vector<V> L((size_t)std::max(n, 1) * n + 1, V(0)), U(L);
+        for (int i = 0; i < n; i++) {
+            for (int j = Lrptr[i]; j < Lrptr[i + 1]; j++) L[(size_t)i * n + Lcind[j]] = Lval[j];
+            for (int j = Urptr[i] + 1; j < Urptr[i + 1]; j++) U[(size_t)i * n + Ucind[j]] = Uval[j];
+        }
+        d.L = dupload(L);
+        d.U = dupload(U);
     }
+    d.dinv = dupload(dinv);
 }
 
 DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval, const int *Urptr,
@@ -1025,43 +1086,46 @@ DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval,
     d.bitL = bitL;
     d.bitU = bitU;
     d.dbitU = dbitU;
-    if (vt == VT_I32) upload_lu_blocks(d, Lrptr, Lcind, (const int32_t *)Lval, Urptr, Ucind, (const int32_t *)Uval);
-    else if (vt == VT_F64) upload_lu_blocks(d, Lrptr, Lcind, (const double *)Lval, Urptr, Ucind, (const double *)Uval);
-    else upload_lu_blocks(d, Lrptr, Lcind, (const float *)Lval, Urptr, Ucind, (const float *)Uval);
+    if (vt == VT_I32) upload_lu(d, Lrptr, Lcind, (const int32_t *)Lval, Urptr, Ucind, (const int32_t *)Uval);
+    else if (vt == VT_F64) upload_lu(d, Lrptr, Lcind, (const double *)Lval, Urptr, Ucind, (const double *)Uval);
+    else upload_lu(d, Lrptr, Lcind, (const float *)Lval, Urptr, Ucind, (const float *)Uval);
     return d;
+}
+
+template <int VT>
+static void launch_chain(Ctx &c, const DevDenseLU &LU, const void *in, void *out) {
+    using V = vt_t<VT>;
+    LuChain<VT> a;
+    a.n = LU.n;
+    a.L = (const V *)LU.Lb;
+    a.U = (const V *)LU.Ub;
+    a.dinv = (const V *)LU.dinv;
+    a.bitL = LU.bitL;
+    a.bitU = LU.bitU;
+    a.dbitU = LU.dbitU;
+    a.in = (const V *)in;
+    a.out = (V *)out;
+    a.ld = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kLuCtas);
+    cfg.blockDim = dim3(32 * kLuWarps);
+    cfg.dynamicSmemBytes = lu_smem<VT>((LU.n + 31) / 32).bytes;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kLuCtas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    SAGB_CUDA(cudaLaunchKernelEx(&cfg, k_lu_chain<VT>, a, c.d_flags));
 }
 
 template <int VT, bool EXACT>
 static void launch_lu(Ctx &c, const DevDenseLU &LU, const void *in, void *out) {
     c.launches++;
-    const int chain = lu_smem<VT>((LU.n + 31) / 32).bytes;
-    if (!EXACT && (VT != VT_I32 || (LU.bitL >= 0 && LU.bitL < 32))) {
-        using V = vt_t<VT>;
-        LuChain<VT> a;
-        a.n = LU.n;
-        a.L = (const V *)LU.L;
-        a.U = (const V *)(kLuScaled<VT> ? LU.W : LU.U);
-        a.dinv = (const V *)LU.dinv;
-        a.bitL = LU.bitL;
-        a.bitU = LU.bitU;
-        a.dbitU = LU.dbitU;
-        a.in = (const V *)in;
-        a.out = (V *)out;
-        a.ld = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kLuCtas);
-        cfg.blockDim = dim3(32 * kLuWarps);
-        cfg.dynamicSmemBytes = chain;
-        cfg.stream = c.stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = kLuCtas;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        SAGB_CUDA(cudaLaunchKernelEx(&cfg, k_lu_chain<VT>, a, c.d_flags));
-        return;
+    if constexpr (!EXACT && VT != VT_F32) {
+        if (chain_takes(VT, LU.bitL)) return launch_chain<VT>(c, LU, in, out);
     }
     const size_t smem = (sizeof(acc_t<VT>) + sizeof(vt_t<VT>)) * (size_t)LU.n;
     k_dense_lu<VT, EXACT><<<1, kLuThreads, smem, c.stream>>>(LU.n, LU.L, LU.U, LU.dinv, LU.bitL, LU.bitU,
@@ -1073,9 +1137,11 @@ static void cta_attrs() {
     const int mx = (int)kSmemMax;
     for (int lg = 0; lg <= 5; lg++)
         for (int lines = 1; lines <= 4; lines *= 2)
-            SAGB_CUDA(cudaFuncSetAttribute(sweep_kernel<VT, EXACT>(lg, lines), cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+            for (int virt = 0; virt <= (VT == VT_F32 && lines == 4 ? std::min(3, 5 - lg) : 0); virt++)
+                SAGB_CUDA(cudaFuncSetAttribute(sweep_kernel<VT, EXACT>(lg, lines, virt), cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     SAGB_CUDA(cudaFuncSetAttribute(k_dense_lu<VT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    if (!EXACT) SAGB_CUDA(cudaFuncSetAttribute(k_lu_chain<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
+    if constexpr (!EXACT && VT != VT_F32)
+        SAGB_CUDA(cudaFuncSetAttribute(k_lu_chain<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
 }
 
 void init_kernel_attributes() {

@@ -126,8 +126,9 @@ Shape pick_shape(const Triangle &A, const std::vector<int> &by_level, const std:
     Shape best;
     best.blocks = P;
     std::vector<double> slowest(kept);
-    for (int lg = 0; lg <= (lim.one_lane ? 0 : 5); lg++)
-        for (int lines = 1; lines <= 4; lines *= 2)
+    // (a lane that stands for several takes eight entries a record, one or more of each)
+    for (int lg = std::max(lim.lanes_log - 3, 0); lg <= (lim.lanes_log >= 0 ? lim.lanes_log : 5); lg++)
+        for (int lines = lg < lim.lanes_log ? 4 : 1; lines <= 4; lines *= 2)
             for (int w = 2; w <= kSweepMaxWarps; w *= 2) {
                 const int per = 32 >> lg, lane = 2 * lines << lg;
                 const double rec = c.record + c.line * lines + (lg == 5 ? c.sum32 : c.round * lg);
@@ -373,6 +374,7 @@ SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, i
     const int P = sh.blocks, W = sh.warps;
     s.lg = sh.lg;
     s.lines = sh.lines;
+    s.virt = lim.lanes_log > sh.lg ? lim.lanes_log - sh.lg : 0;
     s.quads = 1 + s.lines + (es == 8);
     s.row0 = cut_rows(rptr, n, P);
     std::vector<unsigned char> exported(n, 0);

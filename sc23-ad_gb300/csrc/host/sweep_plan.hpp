@@ -40,7 +40,7 @@ struct SweepLimits {
     int sms = 1;                 // CTAs that run at the same time
     int smem = 0;                // bytes of shared memory of a CTA
     bool integer = false;        // 4-byte integers (else floating point)
-    bool one_lane = false;       // one lane a row (sums in the row's order)
+    int lanes_log = -1;          // log2 of a row's lanes where the order of its sum is given
 };
 
 constexpr int kSweepImporters = 8;   // most warps that fetch imports (a power of two)
@@ -58,6 +58,7 @@ struct SweepPlan {
     int n = 0, nlev = 0, max_level_rows = 0;
     int64_t nnz_off = 0;
     int blocks = 0, warps = 0, importers = 0, lg = 0, lines = 0, quads = 0;  // importers: a power of two
+    int virt = 0;  // each lane stands for 2^virt (SweepLimits::lanes_log)
     int max_slots = 0;                    // largest block (rows, imports, zero and spare)
     std::vector<int> row0;                // first row of each block (blocks + 1)
     std::vector<int> steps;               // steps (and barriers) of each block

@@ -86,6 +86,7 @@ struct DevCsr {
     int bit = 0;
     int vt = VT_I32;
     int group = 1;  // lanes per row in the SpMV kernel
+    int lanes = 0;  // FP32: lanes whose order of a row's sum is kept
     int *rptr = nullptr, *cind = nullptr;
     void *val = nullptr;
     void release();
@@ -131,7 +132,7 @@ struct DevTri {
     void *blocks = nullptr, *data = nullptr;
     long long *stream = nullptr;
     int *imp_place = nullptr, *grp = nullptr;
-    int warps = 0, importers = 0, lg = 0, lines = 0;
+    int warps = 0, importers = 0, lg = 0, lines = 0, virt = 0;
     size_t smem = 0;
     void release();
 };
@@ -153,12 +154,13 @@ void trsv(Ctx &c, const DevTri &T, const void *in, void *out);
 // the same sweep with its scratch in a static device array (no allocation)
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out);
 
-// Dense coarsest-level LU: strict lower L (unit) and strict upper U as 32 x 32
-// blocks of the triangles (cuda/lu_chain.cuh), and D^-1; FP64 also U D^-1.
+// Dense coarsest-level LU: strict lower L (unit), strict upper U and D^-1, as the
+// kernels take them (cuda/trsv.cu): L and U row by row, Lb and Ub in 32 x 32 blocks
+// of the triangles (cuda/lu_chain.cuh; FP64: Ub is U D^-1).
 struct DevDenseLU {
     int n = 0, vt = VT_I32;
     int bitL = 0, bitU = 0, dbitU = 0;
-    void *L = nullptr, *U = nullptr, *W = nullptr, *dinv = nullptr;
+    void *L = nullptr, *U = nullptr, *Lb = nullptr, *Ub = nullptr, *dinv = nullptr;
     void release();
 };
 DevDenseLU upload_dense_lu(const int *Lrptr, const int *Lcind, const void *Lval, const int *Urptr,
