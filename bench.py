@@ -509,7 +509,7 @@ def plain_row(ctx, a, r, c, v, b, nrm_b):
     row["coarse_lu_ms"] = k["coarse_lu"]["ms"]
     row["sweep_levels"] = [(p["level"], p["n"], p["levels"], round(p["ms"], 4)) for p in k["sweeps"]["per_level"]]
     l0 = k["sweeps"]["per_level"][0]
-    row["sweep_level0"] = {"ms": l0["ms"], "bytes": l0["bytes"], "traffic": ncu_traffic("k_tri_level0")}
+    row["sweep_level0"] = {"ms": l0["ms"], "bytes": l0["bytes"], "traffic": ncu_traffic("k_sweep_level0")}
     row["spmv_A0"] = k["spmv_A0"]
     S.close()
     S64 = sagb.Solver(ctx, sagb.F64, dA, dA, M64, sagb.solver_params(m=a.m, explicit_stop=1))
