@@ -211,6 +211,8 @@ static void dispatch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mod
             if constexpr (g <= 4)
                 if (A.lanes == 8 * g) return launch_fp<T, g, false, 8>(c, A, x, y, mode, z);
         }
+        // (any other sum would have another order)
+        if (A.lanes && A.lanes != g) throw CudaError{"no SpMV kernel for this number of lanes"};
         launch_fp<T, g, false>(c, A, x, y, mode, z);
     };
     switch (A.group) {
@@ -223,8 +225,7 @@ static void dispatch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mod
     }
 }
 
-void spmv(Ctx &c, const DevCsr &A_, const void *x, void *y, int mode, const void *z) {
-    DevCsr A = A_; if (const char *e = getenv("SAGB_GRP")) A.group = atoi(e);
+void spmv(Ctx &c, const DevCsr &A, const void *x, void *y, int mode, const void *z) {
     if (A.vt == VT_I32) {
         switch (A.group) {
             case 1: return launch_i32<1>(c, A, x, y, mode, z);
