@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <stdexcept>
 
+#include "../host/spmv_lanes.hpp"
 #include "../sagb_internal.hpp"
 #include "common.cuh"
 #include "rows.cuh"
@@ -37,26 +38,6 @@ void DevCsr::release() {
     val = nullptr;
 }
 
-// Lanes per row of the plain SpMV: a twelfth of the average row, so that a lane
-// has several entries in flight and a warp reads few lines at a time, and more in
-// matrices too small to fill the chip that way (up to about a row's entries:
-// there the longest row counts).  Measured us by lanes, 1 / 2 / 4 / 8 / 16 / 32:
-//   FP64 2.05 M rows of 7:    39.6 / 62 / 79 / 133 / 317 / 747
-//   FP64 250 k rows of 55:    60 / 44 / 41 / 65 / 83 / 110
-//   int 250 k rows of 55:     42 / 28 / 26 / 30 / 39 / 58
-//   int 125 k rows of 81:     42 / 26 / 24 / 19 / 22 / 31
-//   FP64 20.8 k rows of 339:  76 / 37 / 27 / 26 / 26 / 28
-//   FP64 2.5 k rows of 258:   71 / 40 / 24 / 14 / 9.9 / 8.7
-// (before: three quarters of the average row, so 4, 32, -, -, 32, 32 of them)
-static int spmv_group(int n, int64_t nnz) {
-    if (n == 0) return 1;
-    const double avg = (double)nnz / n;
-    int g = 1;
-    while (g < 32 && avg > 12 * 1.414 * g) g *= 2;
-    while (g < 32 && (int64_t)n * g < 131072 && g < 0.75 * avg) g *= 2;
-    return g;
-}
-
 int pick_group(double avg) {
     // lanes per row: about the average row length, within [1, 32]
     int g = 1;
@@ -74,7 +55,7 @@ DevCsr upload_csr_i32(const CsrI &A) {
     d.rptr = dupload(A.rptr);
     d.cind = A.cind.empty() ? (int *)dmalloc(16) : dupload(A.cind);
     d.val = A.val.empty() ? dmalloc(16) : (void *)dupload(A.val);
-    d.group = spmv_group(A.n, d.nnz);
+    d.group = spmv_lanes(A.n, d.nnz, longest_row(A.rptr.data(), A.n));
     return d;
 }
 
@@ -88,11 +69,10 @@ DevCsr upload_csr_fp(const CsrT<T> &A) {
     d.rptr = dupload(A.rptr);
     d.cind = A.cind.empty() ? (int *)dmalloc(16) : dupload(A.cind);
     d.val = A.val.empty() ? dmalloc(16) : (void *)dupload(A.val);
-    d.group = spmv_group(A.n, d.nnz);
-    if (d.vt == VT_F32) {  // the row's sum as by d.lanes lanes (see row_part_of)
-        d.lanes = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
-        d.group = std::min(std::max(d.group, d.lanes / 8), d.lanes);
-    }
+    // FP32: the row's sum as by d.lanes lanes (see row_part_of)
+    if (d.vt == VT_F32) d.lanes = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
+    d.group = spmv_lanes(A.n, d.nnz, longest_row(A.rptr.data(), A.n), d.lanes ? d.lanes : 32);
+    if (d.lanes) d.group = std::max(d.group, d.lanes / 8);
     return d;
 }
 template DevCsr upload_csr_fp<double>(const CsrT<double> &);
@@ -107,7 +87,7 @@ DevCsr upload_csr_f64(const CsrD &A) {
     d.rptr = dupload(A.rptr);
     d.cind = dupload(A.cind);
     d.val = dupload(A.val);
-    d.group = spmv_group(A.n, d.nnz);
+    d.group = spmv_lanes(A.n, d.nnz, longest_row(A.rptr.data(), A.n));
     return d;
 }
 
