@@ -17,7 +17,7 @@ OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libsagb.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-HOST_SRC = ["host/amg_setup.cpp", "host/schedule.cpp", "host/sweep_plan.cpp", "host/generators.cpp", "host/features.cpp",
+HOST_SRC = ["host/amg_setup.cpp", "host/schedule.cpp", "host/sweep_plan.cpp", "host/tri_cost.cpp", "host/generators.cpp", "host/features.cpp",
             "host/batch_setup.cpp"]
 CUDA_SRC = ["cuda/spmv.cu", "cuda/trsv.cu", "cuda/amg.cu", "cuda/krylov.cu", "cuda/mlp.cu", "cuda/batch.cu", "cuda/batch_fp.cu",
             "cuda/rs_setup.cu", "capi.cu"]

@@ -9,15 +9,24 @@
 // level only reads rows of earlier levels, so computing level after level gives
 // the integer results of the sequential loop.
 //
-// Two kernels:
+// Three kernels, picked at upload by what they are expected to take
+// (host/sweep_plan.cpp, host/tri_cost.hpp):
 //  * k_sweep: contiguous blocks of rows, one CTA each, the block's values in
-//    shared memory, every level's row data streamed ahead by bulk copies; one
-//    block where the vector fits one CTA's shared memory and the levels are
-//    small.  It needs every row of a block to read rows of the same or of
-//    earlier blocks.
-//  * k_tri (what k_sweep's plan cannot hold: large multicolour sweeps, whose
-//    rows also read later rows, and triangles that reach back too far for the
-//    shared memory): one CTA per SM claims chunks of level-ordered rows
+//    shared memory, every level's row data copied ahead by the lanes that use
+//    them; one block where the vector fits one CTA's shared memory and the
+//    levels are small.  It needs every row of a block to read rows of the same
+//    or of earlier blocks.
+//  * k_tri_cta (few levels of many rows, the vector fits in shared memory): one
+//    CTA.  The result vector lives in shared memory, seeded with `in` (a row
+//    reads its own input once and then overwrites it).  Each level's row data
+//    is one 16-byte aligned block that a bulk copy (cp.async.bulk + mbarrier)
+//    brings into a byte ring in shared memory (all of it not taken by the
+//    vector) up to kCtaSlots levels ahead, so a level costs shared memory
+//    traffic and one block barrier.
+//  * k_tri (few levels of many rows in larger triangles; what k_sweep's plan
+//    cannot hold: large multicolour sweeps, whose rows also read later rows,
+//    and triangles that reach back too far for the shared memory): one CTA per
+//    SM claims chunks of level-ordered rows
 //    by ticket; a row waits only for the rows it reads.  Integer and FP32
 //    results are published as one 64-bit word {epoch, value}, so a dependency
 //    costs one L2 load; FP64 results use an epoch flag with release/acquire.
@@ -25,7 +34,7 @@
 //    not yet published.  Chunks are claimed in level order and depend only on
 //    earlier chunks, so the waits cannot deadlock.
 // All waits are bounded in time (ST_TIMEOUT); ticket and epoch are advanced by
-// the last CTA, so both kernels replay from a CUDA graph.
+// the last CTA, so all of them replay from a CUDA graph.
 #include <algorithm>
 #include <cstring>
 #include <exception>
@@ -42,9 +51,7 @@
 
 namespace sagb {
 
-constexpr int kTriThreads = 256;   // multi-CTA kernel
-constexpr int kBatch = 4;          // dependencies read together per lane (multi-CTA)
-
+constexpr int kBatch = kTriBatch;  // dependencies read together per lane (k_tri)
 
 __device__ __forceinline__ bool aborted(const unsigned *flags) {
     return (*(volatile const unsigned *)flags & ST_TIMEOUT) != 0;
@@ -204,6 +211,202 @@ __global__ void __launch_bounds__(kTriThreads) k_tri(TriArgs a, const void *in, 
             st_release_u32(&a.sync->epoch, ep);
         }
     }
+}
+
+// ============================================================= single CTA
+//
+// Level block (host layout, 16-byte aligned, size a multiple of 16):
+//   int32 header[8] = {R, E, off_val, off_dinv, off_perm, off_rp, 0, 0}
+//   val[E] (V), dinv[R] (V), perm[R], rp[R+1] (0-based inside the block), pci[E]
+
+template <int VT, int G, bool EXACT>
+__device__ __forceinline__ void cta_level(const unsigned char *blk, vt_t<VT> *s_out, int bit, int dbit, int warp,
+                                          int sub, int g, bool &ovf) {
+    using V = vt_t<VT>;
+    constexpr int RPW = 32 / G;
+    constexpr int NW = kCtaThreads / 32 - 1;  // the last warp issues the bulk copies
+    const int *hdr = (const int *)blk;
+    const int R = hdr[0];
+    const V *val = (const V *)(blk + hdr[2]);
+    const V *dv = (const V *)(blk + hdr[3]);
+    const int *perm = (const int *)(blk + hdr[4]);
+    const int *rp = (const int *)(blk + hdr[5]);
+    const int *pci = rp + R + 1;
+    for (int base = warp * RPW; base < R; base += NW * RPW) {
+        const int r = base + sub;
+        const bool valid = r < R;
+        acc_t<VT> t = 0;
+        int row = 0;
+        if (valid) {
+            row = perm[r];
+            const int jb = rp[r], je = rp[r + 1];
+            if (g == 0) t = acc_init<VT>(s_out[row], bit);
+            // four entries of the lane at a time: their loads are issued
+            // together, the products are taken in the lane's order
+            int j = jb + g;
+            for (; j + 3 * G < je; j += 4 * G) {
+                const int c0 = pci[j], c1 = pci[j + G], c2 = pci[j + 2 * G], c3 = pci[j + 3 * G];
+                const V v0 = val[j], v1 = val[j + G], v2 = val[j + 2 * G], v3 = val[j + 3 * G];
+                const V o0 = s_out[c0], o1 = s_out[c1], o2 = s_out[c2], o3 = s_out[c3];
+                t = acc_sub<VT, EXACT>(t, v0, o0);
+                t = acc_sub<VT, EXACT>(t, v1, o1);
+                t = acc_sub<VT, EXACT>(t, v2, o2);
+                t = acc_sub<VT, EXACT>(t, v3, o3);
+            }
+            for (; j < je; j += G) t = acc_sub<VT, EXACT>(t, val[j], s_out[pci[j]]);
+        }
+        t = acc_reduce<VT>(t, G);
+        if (valid && g == 0) s_out[row] = acc_finish<VT>(t, dv[r], bit, dbit, ovf);
+    }
+}
+
+// Shared memory of the single-CTA kernel: the result vector, a byte ring for
+// the level blocks, kCtaSlots mbarriers, the ring position of each level in
+// flight, the block offsets and the rows of each level.  The first lane of
+// the last warp (the producer; that warp computes no rows, so issuing copies
+// never delays a level) places every block contiguously in the ring, in level
+// order (at the write position, or at the ring's start when the end has no
+// room), as soon as the ring has room and fewer than kCtaSlots levels are in
+// flight; a block larger than the whole ring is read from global memory
+// instead.  Level d is always placed by the time the CTA reaches it: the
+// producer places it right after the barrier of level d-1 at the latest, when
+// every earlier level has been consumed and the ring is empty.
+//
+// (A variant without the barrier per level, each row waiting on done bits of
+// the rows it reads, ran about twice as slow on the coarse levels of Poisson
+// 128^3: the waiting rows' shared-memory polling slowed the rows being
+// computed more than the barrier costs.)
+template <int VT, int G, bool EXACT>
+__global__ void __launch_bounds__(kCtaThreads, 1)
+k_tri_cta(const unsigned char *__restrict__ blocks, const unsigned *__restrict__ blk_off, int nlev, int n,
+          int bit, int dbit, int ring_bytes, const void *in_, void *out_, unsigned *flags) {
+    using V = vt_t<VT>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    V *s_out = (V *)smem_raw;
+    const size_t vec_bytes = ((size_t)n * sizeof(V) + 15) & ~(size_t)15;
+    unsigned char *ring = smem_raw + vec_bytes;
+    unsigned long long *bar = (unsigned long long *)(ring + ring_bytes);
+    unsigned *s_pos = (unsigned *)(bar + kCtaSlots);  // ring offset of each level in flight
+    unsigned *s_off = s_pos + kCtaSlots;              // block offsets in 16-byte units
+    const unsigned *s_rows = s_off + nlev + 1;     // rows of each level
+    const V *in = (const V *)in_;
+    V *out = (V *)out_;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane % G, sub = lane / G;
+    constexpr int kProducerWarp = kCtaThreads / 32 - 1;
+    const bool compute = warp != kProducerWarp;
+    const bool producer = warp == kProducerWarp && lane == 0;
+    bool ovf = false;
+
+    if (producer) {
+        for (int s = 0; s < kCtaSlots; s++) mbar_init(bar + s, 1);
+        fence_mbar_init();
+    }
+    for (int i = threadIdx.x; i < n; i += kCtaThreads) s_out[i] = in[i];
+    for (int i = threadIdx.x; i <= 2 * nlev; i += kCtaThreads) s_off[i] = __ldg(blk_off + i);
+    __syncthreads();
+    auto bytes_of = [&](int d) { return (s_off[d + 1] - s_off[d]) * 16u; };
+    auto staged = [&](int d) { return bytes_of(d) <= (unsigned)ring_bytes; };
+    // the producer's ring state: levels [consumed, issued) are in flight; the
+    // nst staged ones among them occupy [lo, head), wrapped once when head <= lo
+    int issued = 0, nst = 0;
+    unsigned lo = 0, head = 0;
+    auto issue_more = [&](int consumed) {  // producer only
+        while (issued < nlev && issued - consumed < kCtaSlots) {
+            const int d = issued;
+            if (staged(d)) {
+                const unsigned b = bytes_of(d);
+                unsigned pos;
+                if (nst == 0) {
+                    pos = 0;
+                    lo = 0;
+                } else if (head > lo) {  // [lo, head): room at the end, else at the start
+                    if (b <= (unsigned)ring_bytes - head) pos = head;
+                    else if (b <= lo) pos = 0;
+                    else break;
+                } else {  // [lo, ring) and [0, head): room between head and lo
+                    if (b <= lo - head) pos = head;
+                    else break;
+                }
+                head = pos + b;
+                nst++;
+                const int s = d % kCtaSlots;
+                // the region's previous readers passed the level barrier
+                // before this copy is issued (no proxy fence is needed for a
+                // bulk copy into memory that generic loads only read)
+                s_pos[s] = pos;  // published to the waiting threads by the arrive below
+                mbar_expect_tx(bar + s, b);
+                bulk_g2s(ring + pos, blocks + (size_t)s_off[d] * 16, b, bar + s);
+            }
+            issued++;
+        }
+    };
+    if (producer) issue_more(0);
+    unsigned phase = 0;  // bit s: parity of slot s's next completion
+    int stuck = -1;      // level whose copy did not arrive in time
+    for (int d = 0; d < nlev; d++) {
+        const bool st = staged(d);
+        const int s = d % kCtaSlots;
+        const unsigned char *blk = blocks + (size_t)s_off[d] * 16;
+        bool timed_out = false;
+        // a warp with no row in this level neither waits for its block nor
+        // reads it (it only keeps the slot parities)
+        constexpr int kRowsPerWarp = 32 / G;
+        const bool mine = compute && warp * kRowsPerWarp < (int)s_rows[d];
+        if (st && !mine) {
+            phase ^= 1u << s;
+        } else if (st) {
+            // bounded wait for the bulk copy of this level
+            const unsigned par = (phase >> s) & 1u;
+            if (!mbar_try_wait(bar + s, par)) {
+                const unsigned long long t0 = globaltimer_ns();
+                while (!mbar_try_wait(bar + s, par)) {
+                    if (globaltimer_ns() - t0 > kSpinLimitNs) {
+                        timed_out = true;
+                        break;
+                    }
+                }
+            }
+            phase ^= 1u << s;
+            blk = ring + s_pos[s];
+        }
+        if (mine && !timed_out) cta_level<VT, G, EXACT>(blk, s_out, bit, dbit, warp, sub, g, ovf);
+        // one barrier per level: results visible, the level's ring space free
+        if (__syncthreads_or(timed_out)) {
+            stuck = d;
+            break;
+        }
+        if (producer) {
+            if (st && --nst > 0) {
+                for (int e = d + 1; e < issued; e++)
+                    if (staged(e)) {
+                        lo = s_pos[e % kCtaSlots];
+                        break;
+                    }
+            }
+            issue_more(d + 1);
+        }
+    }
+    if (stuck >= 0) {
+        // report, then wait (bounded) for the copies this CTA still has in
+        // flight before its shared memory goes away
+        if (producer) {
+            atomicOr(flags, ST_TIMEOUT);
+            const unsigned long long t0 = globaltimer_ns();
+            for (int dd = stuck; dd < issued; dd++) {
+                if (!staged(dd)) continue;
+                const int s = dd % kCtaSlots;
+                // the stuck level's wait already flipped its parity bit
+                const unsigned par = ((phase >> s) & 1u) ^ (dd == stuck ? 1u : 0u);
+                while (!mbar_try_wait(bar + s, par) && globaltimer_ns() - t0 < kSpinLimitNs) {
+                }
+            }
+        }
+        __syncthreads();
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += kCtaThreads) out[i] = s_out[i];
+    if (ovf) atomicOr(flags, ST_OVERFLOW);
 }
 
 // ================================================================ blocks
@@ -609,12 +812,14 @@ void DevTri::release() {
     if (!blocks) dfree(sync);  // (a sweep by blocks: behind pk; its small arrays: behind blocks)
     dfree(blocks);
     dfree(data);
+    dfree(blk_off);
     perm = prp = pci = chunk_lv = sub_bound = nullptr;
     pval = dinv = nullptr;
     pk = nullptr;
     flag = nullptr;
     sync = nullptr;
     blocks = data = nullptr;
+    blk_off = nullptr;
     stream = nullptr;
     imp_place = grp = nullptr;
 }
@@ -628,39 +833,77 @@ static void gather_vals(const TriSchedule &s, const T *vals, std::vector<T> &pv,
         if (s.diag_src[p] >= 0) dv[p] = vals[s.diag_src[p]];
 }
 
+static size_t up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// one block per level (see the layout above k_tri_cta)
+template <typename T>
+static void build_blocks(const TriSchedule &s, const std::vector<T> &pv, const std::vector<T> &dv,
+                         std::vector<unsigned char> &blob, std::vector<long long> &off) {
+    off.assign(s.nlev + 1, 0);
+    blob.clear();
+    for (int l = 0; l < s.nlev; l++) {
+        const int p0 = s.lvl_ptr[l], p1 = s.lvl_ptr[l + 1];
+        const int R = p1 - p0;
+        const int e0 = s.prp[p0], e1 = s.prp[p1];
+        const int E = e1 - e0;
+        const size_t o_val = 32;
+        const size_t o_dinv = up(o_val + sizeof(T) * E, 8);
+        const size_t o_perm = up(o_dinv + sizeof(T) * R, 4);
+        const size_t o_rp = o_perm + 4 * (size_t)R;
+        const size_t o_pci = o_rp + 4 * (size_t)(R + 1);
+        const size_t size = up(o_pci + 4 * (size_t)E, 16);
+        const size_t base = blob.size();
+        blob.resize(base + size, 0);
+        unsigned char *b = blob.data() + base;
+        int hdr[8] = {R, E, (int)o_val, (int)o_dinv, (int)o_perm, (int)o_rp, 0, 0};
+        memcpy(b, hdr, sizeof hdr);
+        memcpy(b + o_val, pv.data() + e0, sizeof(T) * E);
+        memcpy(b + o_dinv, dv.data() + p0, sizeof(T) * R);
+        memcpy(b + o_perm, s.perm.data() + p0, 4 * (size_t)R);
+        int *rp = (int *)(b + o_rp);
+        for (int r = 0; r <= R; r++) rp[r] = s.prp[p0 + r] - e0;
+        memcpy(b + o_pci, s.pci.data() + e0, 4 * (size_t)E);
+        off[l + 1] = (long long)blob.size();
+    }
+}
+
 static int pow2_at_least(double x) {
     int g = 1;
     while (g < 32 && g < x) g <<= 1;
     return g;
 }
 
+// Lanes a row in k_tri_cta and k_tri: a quarter of its average length (off the
+// diagonal), one in the sequential-order mode.
+constexpr int kRowShare = 4;
+static int tri_lanes(const Ctx &c, const TriSource &t, int vt) {
+    if (vt != VT_I32 && c.fp_exact) return 1;
+    return pow2_at_least((t.n ? ((double)t.rptr[t.n] - t.n) / t.n : 0.0) / kRowShare);
+}
+
 // Lanes a row where its sum has one order: one in the sequential-order mode.  FP32
 // solves converge in a number of iterations that follows the last bits of their
-// V-cycles, so an FP32 row is summed by both kernels by a number of lanes that
-// depends on its triangle alone: lane g takes entries g, g + G, ... in their order,
+// V-cycles, so an FP32 row is summed by all kernels as by tri_lanes lanes, which
+// depend on its triangle alone: lane g takes entries g, g + G, ... in their order,
 // lane 0 starts from the input, and the lanes are added by a butterfly.  k_sweep may
 // let a lane stand for up to eight of them.  (Lanes and order free, and the coarsest
 // solve on the cluster: an FP32 V-cycle of a 383^2 grid with 40 blocks 714 us
 // instead of 910; but solves of 27-point and variable-coefficient systems took
 // another number of iterations or ended 1e-8 apart.)
-static int fixed_lanes(const Ctx &c, int vt, int n, int64_t off) {
-    if (vt == VT_I32) return 0;
-    if (c.fp_exact) return 1;
-    if (vt == VT_F64) return 0;
-    return pow2_at_least((n ? (double)off / n : 0.0) / ((size_t)n * 4 <= 150 * 1024 ? 4 : kBatch));
-}
+static bool fixed_order(const Ctx &c, int vt) { return vt == VT_F32 || (vt == VT_F64 && c.fp_exact); }
 
 static SweepPlan plan_tri(const Ctx &c, const TriSource &t, int vt) {
     SweepLimits lim;
     lim.sms = c.num_sms;
     lim.smem = (int)kSmemMax;
     lim.integer = vt == VT_I32;
-    if (const int g = fixed_lanes(c, vt, t.n, t.n ? (int64_t)t.rptr[t.n] - t.n : 0)) lim.lanes_log = __builtin_ctz(g);
+    lim.lanes = tri_lanes(c, t, vt);
+    if (fixed_order(c, vt)) lim.lanes_log = __builtin_ctz(lim.lanes);
     return build_sweep_plan(t.rptr, t.cind, t.vals, (int)vt_size(vt), t.n, lim, t.level_hint);
 }
 
 static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const SweepPlan &p) {
-    const int n = src.n, *rptr = src.rptr, *cind = src.cind;
+    const int n = src.n;
     const void *vals = src.vals;
     DevTri d;
     d.n = n;
@@ -710,25 +953,41 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
         }
         return d;
     }
-    const double avg = n ? (double)d.nnz_off / n : 0.0;
-    const int fixed = fixed_lanes(c, vt, n, d.nnz_off), G = fixed ? fixed : pow2_at_least(avg / kBatch);
-    d.group = G;
-    const int rows_per_chunk = 2 * kTriThreads / G;
-    TriSchedule s = build_tri_schedule(rptr, cind, n, TRI_LD, rows_per_chunk, 1 << 20, src.level_hint);
+    const TriSchedule &s = *p.levels;
+    d.group = tri_lanes(c, src, vt);
+    d.one_cta = p.one_cta;
     d.nlev = s.nlev;
     d.max_level_rows = s.max_level_rows;
     d.nnz_off = (int64_t)s.pci.size();
     d.nchunks = s.nchunks();
+    std::vector<unsigned char> blob;
+    std::vector<long long> off;
     auto put_vals = [&](auto tag) {
         using T = decltype(tag);
         std::vector<T> pv, dv;
         gather_vals(s, (const T *)vals, pv, dv);
-        d.pval = pv.empty() ? dmalloc(16) : (void *)dupload(pv);
-        d.dinv = dupload(dv);
+        if (d.one_cta) {
+            build_blocks(s, pv, dv, blob, off);
+        } else {
+            d.pval = pv.empty() ? dmalloc(16) : (void *)dupload(pv);
+            d.dinv = dupload(dv);
+        }
     };
     if (vt == VT_I32) put_vals(int32_t());
     else if (vt == VT_F64) put_vals(double());
     else put_vals(float());
+    if (d.one_cta) {
+        d.blocks = blob.empty() ? dmalloc(16) : (void *)dupload(blob);
+        // block offsets in 16-byte units (nlev + 1), then the rows of each level (nlev)
+        std::vector<unsigned> off16(off.size() + s.nlev);
+        for (size_t i = 0; i < off.size(); i++) off16[i] = (unsigned)(off[i] / 16);
+        for (int l = 0; l < s.nlev; l++) off16[off.size() + l] = (unsigned)(s.lvl_ptr[l + 1] - s.lvl_ptr[l]);
+        d.blk_off = dupload(off16);
+        d.stage_bytes = (int)((kSmemMax - cta_fixed_smem(n, (int)vt_size(vt), s.nlev)) / 16 * 16);
+        d.smem = cta_fixed_smem(n, (int)vt_size(vt), s.nlev) + (size_t)d.stage_bytes;
+        d.grid = 1;
+        return d;
+    }
     d.perm = dupload(s.perm);
     d.prp = dupload(s.prp);
     d.pci = s.pci.empty() ? (int *)dmalloc(16) : dupload(s.pci);
@@ -780,10 +1039,15 @@ std::vector<DevTri> upload_tris(const Ctx &c, const std::vector<TriSource> &src,
 
 template <int VT, int G, bool EXACT>
 static void launch_tri(Ctx &c, const DevTri &T, const void *in, void *out) {
+    c.launches++;
+    if (T.one_cta) {
+        k_tri_cta<VT, G, EXACT><<<1, kCtaThreads, T.smem, c.stream>>>((const unsigned char *)T.blocks, T.blk_off, T.nlev, T.n, T.bit,
+                                                                      T.dbit, T.stage_bytes, in, out, c.d_flags);
+        return;
+    }
     TriArgs a{T.n, T.nchunks, T.bit, T.dbit, T.perm, T.prp, T.pci, T.pval, T.dinv,
               T.chunk_lv, T.sub_bound, T.pk, T.flag, T.sync};
     k_tri<VT, G, EXACT><<<T.grid, kTriThreads, 0, c.stream>>>(a, in, out, c.d_flags);
-    c.launches++;
 }
 
 using SweepKernel = void (*)(SweepArgs, const void *, void *, unsigned *);
@@ -813,7 +1077,7 @@ static SweepKernel sweep_kernel(int lg, int lines, int virt) {
 
 template <int VT, bool EXACT>
 static void tri_by_group(Ctx &c, const DevTri &T, const void *in, void *out) {
-    if (T.blocks) {
+    if (T.data) {
         int ilog = 0;
         while (2 << ilog <= T.importers) ilog++;
         SweepArgs a{T.warps, ilog, T.bit, T.dbit, (const SweepBlock *)T.blocks, T.stream, (const uint4 *)T.data, T.imp_place,
@@ -883,7 +1147,7 @@ static unsigned long long *noalloc_scratch(int device) {
 }
 
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
-    if (T.n == 0 || (T.blocks && T.grid == 1)) return trsv(c, T, in, out);  // shared memory only: no scratch
+    if (T.n == 0 || T.one_cta || (T.data && T.grid == 1)) return trsv(c, T, in, out);  // shared memory only: no scratch
     if (T.n > kNoAllocRows)
         throw CudaError{"level has more than 262144 rows, the limit of the no-allocation sweep"};
     unsigned long long *s = noalloc_scratch(c.device);
@@ -1139,6 +1403,12 @@ static void cta_attrs() {
         for (int lines = 1; lines <= 4; lines *= 2)
             for (int virt = 0; virt <= (VT == VT_F32 && lines == 4 ? std::min(3, 5 - lg) : 0); virt++)
                 SAGB_CUDA(cudaFuncSetAttribute(sweep_kernel<VT, EXACT>(lg, lines, virt), cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 1, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 2, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 4, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 8, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 16, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    SAGB_CUDA(cudaFuncSetAttribute(k_tri_cta<VT, 32, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     SAGB_CUDA(cudaFuncSetAttribute(k_dense_lu<VT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     if constexpr (!EXACT && VT != VT_F32)
         SAGB_CUDA(cudaFuncSetAttribute(k_lu_chain<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));

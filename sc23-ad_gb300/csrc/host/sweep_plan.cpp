@@ -67,13 +67,28 @@ constexpr double kCostSlot = 4.8;   // shared memory: each entry of a lane, over
 constexpr double kCostImport = 84;  // a step that waits for imports
 constexpr double kCostFetch = 1.5;  // an import
 constexpr double kCostHop = 1490;   // a value published by one block and used by the next (0.8 us)
-constexpr double kCostTri = 7000;   // a level of k_tri
 constexpr double kCostBytes = 21;   // bytes of records one CTA streams a cycle (40 GB/s)
 
 struct Shape {
     int blocks = 0, warps = 1, lg = 0, lines = 1;
     double cost = 1e300;
+    double queued = 0;  // records after the third of a warp and step, in the slowest block of each step
 };
+
+// A shape's time in us, to compare it with the other kernels': the launch, the
+// cycles, and what the model above leaves out because it hardly differs between
+// shapes: a step with many records a warp waits for their copies, of which
+// kSweepStage - 1 are on their way.
+double sweep_us(const Shape &s, int es, bool integer) {
+    const double cycles = es == 8 ? 1.0 : integer ? 0.87 : 0.66, record = es == 8 ? 0.11 : integer ? 0.053 : 0.031;
+    return 4.3 + cycles * s.cost / 1900 + record * s.queued;
+}
+// The estimates are 10 to 15 % off, so k_tri_cta, where the vector fits it, and k_tri
+// elsewhere are left where another kernel promises 12 % less (k_tri for k_tri_cta: 20 %,
+// its estimate is the roughest).  Over the levels that the estimates were fitted to, the
+// kernel picked then took at most 1.13 times as long as the one left, but for one level
+// of 1.27.
+constexpr double kCostMargin = 0.88, kCostSpread = 1.1;
 
 // first row of each of P blocks: rows weighted by their entries and three more
 std::vector<int> cut_rows(const int *rptr, int n, int P) {
@@ -157,6 +172,14 @@ Shape pick_shape(const Triangle &A, const std::vector<int> &by_level, const std:
                     best.lines = lines;
                 }
             }
+    const int per = 32 >> best.lg, lane = 2 * best.lines << best.lg;
+    std::fill(slowest.begin(), slowest.end(), 0.0);
+    for (const Step &q : steps) {
+        const int tasks = (q.rows + per - 1) / per, first = std::max(1, (q.longest + lane - 1) / lane);
+        const double rest = std::max(1.0, (double)q.entries / q.rows / lane);
+        slowest[q.level] = std::max(slowest[q.level], first + ((tasks + best.warps - 1) / best.warps - 1) * rest);
+    }
+    for (double v : slowest) best.queued += std::max(0.0, v - (kSweepStage - 1)) * nlev / kept;
     return best;
 }
 
@@ -320,13 +343,22 @@ SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, i
         s.nlev = std::max(s.nlev, (level_hint ? level_hint[i] : lv) + 1);
         s.nnz_off += A.len(i);
     }
-    if (!lower && !level_hint) return s;  // not a lower triangle
+    // the rows level by level for the kernels that go that way
+    auto by_levels = [&]() -> const TriSchedule & {
+        s.levels.reset(new TriSchedule(build_tri_schedule(rptr, cind, n, TRI_LD, 2 * kTriThreads / lim.lanes, 1 << 20, level_hint)));
+        return *s.levels;
+    };
+    const bool one_cta = cta_fits(n, es, s.nlev, lim.smem);
+    if (n == 0 || (!lower && !level_hint)) {  // (not a lower triangle)
+        by_levels();
+        s.one_cta = one_cta;
+        return s;
+    }
     {
         std::vector<int> count(s.nlev, 0);
         for (int i = 0; i < n; i++)
             s.max_level_rows = std::max(s.max_level_rows, ++count[level_hint ? level_hint[i] : level[i]]);
     }
-    if (n == 0) return s;
     // the steps follow the dependencies themselves where rows read earlier rows
     // only (chunks of rows: fewer levels than chunks), else the hint
     if (!lower) {
@@ -367,10 +399,22 @@ SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, i
     Shape sh;
     for (const Shape &q : shapes)
         if (q.blocks > 0 && q.cost < sh.cost) sh = q;
-    // few levels of many rows (colours, chunks): k_tri spreads a level over all
-    // SMs and takes 3.7 us or more for it (Poisson 60^3, level 2, 27,000 rows in
-    // 23 colours: 155 us in one block, 85 us there)
-    if (sh.blocks == 0 || sh.cost > kCostTri * nlev) return s;
+    // Few levels of many rows (colours, chunks, orders with short chains): a level is
+    // work for more warps than a block has (k_tri_cta: 31) or for all SMs (k_tri).  us
+    // by blocks / one CTA / all SMs: int 4,900 rows in two colours 12.0 / 6.7 / 8.0,
+    // 45,000 rows in four 74 / - / 17; FP64 10,388 rows in 17 colours 116 / 104 / 496,
+    // 98,769 rows in 83 chunks 182 / - / 1,895.
+    const double by_blocks = sh.blocks ? sweep_us(sh, es, lim.integer) : 1e300;
+    const double bias = one_cta ? kCostSpread : kCostMargin;
+    if (by_blocks >= bias * spread_least_us(nlev, es) || (one_cta && by_blocks >= kCostMargin * cta_least_us(s.nlev, es))) {
+        const TriSchedule &t = by_levels();
+        const double cta = one_cta ? kCostMargin * cta_us(t, lim.lanes, es) : 1e300;
+        const double spread = !one_cta && sh.blocks == 0 ? 0.0 : bias * spread_us(t, lim.lanes, es, lim.sms);
+        s.one_cta = cta <= spread;
+        if (std::min(cta, spread) <= by_blocks) return s;
+        s.one_cta = false;
+        s.levels.reset();
+    }
     const int P = sh.blocks, W = sh.warps;
     s.lg = sh.lg;
     s.lines = sh.lines;
@@ -409,7 +453,11 @@ SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, i
         s.max_slots = std::max(s.max_slots, q.b1 - q.b0 + (int)q.imports.size() + 2);
         for (const auto &w : q.records) s.stream.push_back(s.stream.back() + (int64_t)w.size());
     }
-    if (s.max_slots > kSweepMaxSlots || (int64_t)s.max_slots * es + sweep_fixed_smem(W, s.quads) > lim.smem) return s;
+    if (s.max_slots > kSweepMaxSlots || (int64_t)s.max_slots * es + sweep_fixed_smem(W, s.quads) > lim.smem) {
+        by_levels();
+        s.one_cta = one_cta;
+        return s;
+    }
     // the records, in pieces of a few hundred
     struct Piece {
         int block, warp, from, to;

@@ -30,6 +30,8 @@
 #include <memory>
 #include <vector>
 
+#include "tri_cost.hpp"
+
 namespace sagb {
 
 struct SweepQuad {
@@ -41,6 +43,7 @@ struct SweepLimits {
     int smem = 0;                // bytes of shared memory of a CTA
     bool integer = false;        // 4-byte integers (else floating point)
     int lanes_log = -1;          // log2 of a row's lanes where the order of its sum is given
+    int lanes = 1;               // a row's lanes in the kernels that go level by level
 };
 
 constexpr int kSweepImporters = 8;   // most warps that fetch imports (a power of two)
@@ -70,14 +73,18 @@ struct SweepPlan {
     std::vector<int> grp_ptr, grp;        // (grp_ptr: blocks + 1; a block's grp has one entry more than groups)
     std::vector<int64_t> stream;          // first record of (block, warp) (blocks * warps + 1)
     std::unique_ptr<SweepQuad[]> data;    // the streams one after the other
+    // without blocks: the rows level by level, for k_tri_cta (one_cta) or k_tri
+    std::unique_ptr<TriSchedule> levels;
+    bool one_cta = false;
     bool ok() const { return blocks > 0; }
 };
 
 // The plan of the LD sweep rptr / cind / vals (off-diagonal entries, then the
 // inverse diagonal last in each row); es: bytes of a value (4 or 8).
 // level_hint (optional): a level per row in which every dependency has a lower
-// level.  Without blocks (ok() false) when a block cannot be made to fit, or
-// when several blocks are needed and some row reads a later one.
+// level.  Without blocks (ok() false) when a block cannot be made to fit, when
+// several blocks are needed and some row reads a later one, or when a kernel that
+// goes level by level costs less.
 SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, int es, int n,
                            const SweepLimits &lim, const int *level_hint = nullptr);
 

@@ -126,7 +126,7 @@ struct DevTri {
     unsigned long long *pk = nullptr;  // packed {epoch, value} per row (int32 / f32; two words per f64 row of a sweep by blocks)
     unsigned *flag = nullptr;          // ready epoch per row (f64)
     TriSync *sync = nullptr;
-    // the sweep by blocks of rows (host/sweep_plan.hpp; blocks null: k_tri):
+    // the sweep by blocks of rows (host/sweep_plan.hpp; `data` null: k_tri_cta or k_tri):
     // grid CTAs of `warps` compute warps and `importers`, 2^lg lanes a row, `lines` pairs of
     // entries a lane and record
     void *blocks = nullptr, *data = nullptr;
@@ -134,6 +134,11 @@ struct DevTri {
     int *imp_place = nullptr, *grp = nullptr;
     int warps = 0, importers = 0, lg = 0, lines = 0, virt = 0;
     size_t smem = 0;
+    // one CTA level by level (k_tri_cta): `blocks` holds each level's row data in one
+    // 16-byte aligned block
+    bool one_cta = false;
+    unsigned *blk_off = nullptr;  // offset of each level's block in 16-byte units (nlev + 1), then the rows of each level (nlev)
+    int stage_bytes = 0;          // bytes of its bulk-copy ring
     void release();
 };
 
