@@ -233,12 +233,13 @@ int sa_amg_sweep(sa_ctx ctx, sa_amg M, int level, const void *in, void *out);
  * they solve -- their GPU memory is already claimed by another allocator (a
  * framework's caching allocator, a fixed pool), or they cannot afford the
  * device-wide synchronisation that allocating and freeing imply.  in and out
- * must be device buffers.  The scratch of a sweep by several CTAs comes from a
- * static device array sized for 262,144 rows (4 MiB, held by every GPU that
- * loads the library until the process exits); a level with more rows is
- * rejected with SA_ERR_ARG.  The first call on a device looks up that array's
- * address, so make the first call before any stream capture.  Every call
- * shares the array: calls that overlap on the GPU race. */
+ * must be device buffers.  Levels whose vectors take at most 150 KiB sweep in the
+ * context's own scratch, like sa_amg_sweep.  The scratch of larger ones comes
+ * from a static device array sized for 262,144 rows (4 MiB, held by every GPU
+ * that loads the library until the process exits); a level with more rows is
+ * rejected with SA_ERR_ARG.  The first of their calls on a device looks up that
+ * array's address, so make it before any stream capture.  They share the array:
+ * such calls that overlap on the GPU race. */
 int sa_amg_sweep_noalloc(sa_ctx ctx, sa_amg M, int level, const void *in, void *out);
 /* direct::LUflex::Solve / LU<T>::Solve   Library/solver/lu.hpp:30-33, 91-94 */
 int sa_amg_coarse_solve(sa_ctx ctx, sa_amg M, const void *in, void *out);

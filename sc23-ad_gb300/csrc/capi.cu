@@ -192,6 +192,8 @@ extern "C" int sa_ctx_create(int device, sa_ctx *out) {
     h->c.d_flags_main = h->c.d_flags;
     h->c.d_flags_prec = h->c.d_flags + 1;
     SAGB_CUDA(cudaMallocHost(&h->c.h_flags, sizeof(unsigned) * 4));
+    h->c.sweep = (SweepScratch *)dmalloc(sizeof(SweepScratch));
+    SAGB_CUDA(cudaMemsetAsync(h->c.sweep, 0, sizeof(SweepScratch), h->c.stream));
     init_kernel_attributes();
     *out = h;
     return SA_OK;
@@ -204,6 +206,7 @@ extern "C" int sa_ctx_destroy(sa_ctx ctx) {
     dfree(ctx->c.stage[0]);
     dfree(ctx->c.stage[1]);
     dfree(ctx->c.d_flags_main);
+    dfree(ctx->c.sweep);
     cudaFreeHost(ctx->c.h_flags);
     cudaStreamDestroy(ctx->c.stream);
     delete ctx;

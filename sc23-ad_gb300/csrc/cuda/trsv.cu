@@ -809,7 +809,7 @@ void DevTri::release() {
     dfree(sub_bound);
     dfree(pk);
     dfree(flag);
-    if (!blocks) dfree(sync);  // (a sweep by blocks: behind pk; its small arrays: behind blocks)
+    if (!data) dfree(sync);  // (a sweep by blocks: behind pk; its small arrays: behind blocks)
     dfree(blocks);
     dfree(data);
     dfree(blk_off);
@@ -907,6 +907,7 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
     const void *vals = src.vals;
     DevTri d;
     d.n = n;
+    d.small = (size_t)n * vt_size(vt) <= kSmallSweep;
     d.kind = TRI_LD;
     d.vt = vt;
     d.bit = src.bit;
@@ -945,7 +946,7 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
         SAGB_CUDA(cudaMemset((unsigned char *)d.data + bytes, 0, pad));
         SAGB_CUDA(cudaMemcpy(d.data, p.data.get(), bytes, cudaMemcpyHostToDevice));
         d.smem = sweep_fixed_smem(p.warps, p.quads) + (size_t)p.max_slots * vt_size(vt);
-        if (p.blocks > 1) {
+        if (p.blocks > 1 && !d.small) {
             const size_t words = (size_t)n * (vt == VT_F64 ? 2 : 1), all = sizeof(unsigned long long) * words + sizeof(TriSync);
             d.pk = (unsigned long long *)dmalloc(all);
             SAGB_CUDA(cudaMemset(d.pk, 0, all));
@@ -993,6 +994,8 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
     d.pci = s.pci.empty() ? (int *)dmalloc(16) : dupload(s.pci);
     d.chunk_lv = dupload(s.chunk_lv);
     d.sub_bound = dupload(s.sub_bound);
+    d.grid = std::max(1, std::min(d.nchunks, c.num_sms));
+    if (d.small) return d;
     if (vt == VT_F64) {
         d.flag = (unsigned *)dmalloc(sizeof(unsigned) * std::max(n, 1));
         SAGB_CUDA(cudaMemset(d.flag, 0, sizeof(unsigned) * std::max(n, 1)));
@@ -1002,7 +1005,6 @@ static DevTri upload_tri(const Ctx &c, const TriSource &src, int vt, const Sweep
     }
     d.sync = (TriSync *)dmalloc(sizeof(TriSync));
     SAGB_CUDA(cudaMemset(d.sync, 0, sizeof(TriSync)));
-    d.grid = std::max(1, std::min(d.nchunks, c.num_sms));
     return d;
 }
 
@@ -1047,6 +1049,11 @@ static void launch_tri(Ctx &c, const DevTri &T, const void *in, void *out) {
     }
     TriArgs a{T.n, T.nchunks, T.bit, T.dbit, T.perm, T.prp, T.pci, T.pval, T.dinv,
               T.chunk_lv, T.sub_bound, T.pk, T.flag, T.sync};
+    if (T.small) {
+        a.pk = c.sweep->pk;
+        a.flag = c.sweep->flag;
+        a.sync = &c.sweep->sync;
+    }
     k_tri<VT, G, EXACT><<<T.grid, kTriThreads, 0, c.stream>>>(a, in, out, c.d_flags);
 }
 
@@ -1082,6 +1089,10 @@ static void tri_by_group(Ctx &c, const DevTri &T, const void *in, void *out) {
         while (2 << ilog <= T.importers) ilog++;
         SweepArgs a{T.warps, ilog, T.bit, T.dbit, (const SweepBlock *)T.blocks, T.stream, (const uint4 *)T.data, T.imp_place,
                     T.grp, T.pk, T.sync};
+        if (T.small) {
+            a.pk = c.sweep->pk;
+            a.sync = &c.sweep->sync;
+        }
         sweep_kernel<VT, EXACT>(T.lg, T.lines, T.virt)<<<T.grid, 32 * (T.warps + T.importers), T.smem,
                                                  c.stream>>>(a, in, out, c.d_flags);
         c.launches++;
@@ -1112,11 +1123,12 @@ void trsv(Ctx &c, const DevTri &T, const void *in, void *out) {
 //
 // For callers that cannot allocate device memory while they solve (their GPU
 // memory is already claimed by another allocator, or they cannot afford the
-// device-wide synchronisation cudaMalloc/cudaFree imply).  The fine-level sweep
-// kernel needs per-row scratch (the packed {epoch, value} words and the
-// ticket/epoch block); this variant takes it from the file-scope array below
-// instead of the schedule's own allocation.  The array is sized for
-// kNoAllocRows rows (two words each for FP64: 4 MiB) and every GPU that loads the library holds it
+// device-wide synchronisation cudaMalloc/cudaFree imply).  A sweep by several CTAs
+// needs per-row scratch (the packed {epoch, value} words and the ticket/epoch
+// block); small levels have their context's (SweepScratch), larger ones take it
+// here from the file-scope array below instead of the schedule's own allocation.
+// The array is sized for kNoAllocRows rows (two words each for FP64: 4 MiB) and
+// every GPU that loads the library holds it
 // until the process exits.  All calls share it and it keeps the last call's
 // contents, so before each call the words of this level's rows and the
 // ticket, done and epoch counters are cleared (a previous call may have left
@@ -1147,7 +1159,7 @@ static unsigned long long *noalloc_scratch(int device) {
 }
 
 void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
-    if (T.n == 0 || T.one_cta || (T.data && T.grid == 1)) return trsv(c, T, in, out);  // shared memory only: no scratch
+    if (T.n == 0 || T.small || (T.data && T.grid == 1)) return trsv(c, T, in, out);  // the context's scratch, or none
     if (T.n > kNoAllocRows)
         throw CudaError{"level has more than 262144 rows, the limit of the no-allocation sweep"};
     unsigned long long *s = noalloc_scratch(c.device);

@@ -11,6 +11,7 @@
 #include "host/batch_setup.hpp"
 #include "host/csr.hpp"
 #include "host/schedule.hpp"
+#include "host/tri_cost.hpp"
 
 namespace sagb {
 
@@ -46,6 +47,9 @@ struct Ctx {
     void *stage[2] = {nullptr, nullptr};
     size_t stage_cap[2] = {0, 0};
     int stage_used = 0;
+    // scratch of the sweeps over small levels (DevTri::small; the context's calls follow
+    // one another, so one is enough)
+    struct SweepScratch *sweep = nullptr;
     std::string err;
 };
 
@@ -113,6 +117,17 @@ void spmv_resid_f64_exact(Ctx &c, const DevCsr &A, const double *x, const double
 struct TriSync {
     unsigned ticket, done, epoch, pad;
 };
+// What the CTAs of a sweep publish values through: words {epoch, value} and ready epochs
+// (see DevTri), and the ticket, done and epoch counters.  Every sweep raises the epoch,
+// so what another one left here is never taken for its own.  Sweeps over vectors of at most
+// kSmallSweep bytes use their context's, so that contexts can sweep the same small
+// levels at the same time; larger levels have their own.
+constexpr size_t kSmallSweep = kCtaVecMax;
+struct SweepScratch {
+    unsigned long long pk[kSmallSweep / 4];
+    unsigned flag[kSmallSweep / 8];
+    TriSync sync;
+};
 
 struct DevTri {
     int n = 0, kind = 0, vt = VT_I32;
@@ -126,6 +141,7 @@ struct DevTri {
     unsigned long long *pk = nullptr;  // packed {epoch, value} per row (int32 / f32; two words per f64 row of a sweep by blocks)
     unsigned *flag = nullptr;          // ready epoch per row (f64)
     TriSync *sync = nullptr;
+    bool small = false;                // pk, flag and sync are the context's
     // the sweep by blocks of rows (host/sweep_plan.hpp; `data` null: k_tri_cta or k_tri):
     // grid CTAs of `warps` compute warps and `importers`, 2^lg lanes a row, `lines` pairs of
     // entries a lane and record
