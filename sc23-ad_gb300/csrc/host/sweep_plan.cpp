@@ -453,7 +453,9 @@ SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, i
         s.max_slots = std::max(s.max_slots, q.b1 - q.b0 + (int)q.imports.size() + 2);
         for (const auto &w : q.records) s.stream.push_back(s.stream.back() + (int64_t)w.size());
     }
-    if (s.max_slots > kSweepMaxSlots || (int64_t)s.max_slots * es + sweep_fixed_smem(W, s.quads) > lim.smem) {
+    const int64_t own = (int64_t)rptr[n] * (4 + es) + 4ll * n, most = std::max(lim.record_bytes, kSweepRecordShare * own);
+    if (s.max_slots > kSweepMaxSlots || (int64_t)s.max_slots * es + sweep_fixed_smem(W, s.quads) > lim.smem ||
+        s.stream.back() * s.quads * 512 > most) {
         by_levels();
         s.one_cta = one_cta;
         return s;

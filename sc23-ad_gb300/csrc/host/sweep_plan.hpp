@@ -44,6 +44,12 @@ struct SweepLimits {
     bool integer = false;        // 4-byte integers (else floating point)
     int lanes_log = -1;          // log2 of a row's lanes where the order of its sum is given
     int lanes = 1;               // a row's lanes in the kernels that go level by level
+    // Records may take this much memory, or kSweepRecordShare times the triangle's own if
+    // that is more.  A record has room for 32 lanes: where a level has one or two rows
+    // (tridiagonal and narrow band matrices) a row takes 1 to 1.5 KiB of it instead of 20
+    // bytes, and a matrix of tens of millions of rows all of a GPU's memory.  (Levels of
+    // 2D and 3D grids: 1.3 to 4 times the triangle, up to 9 where small.)
+    int64_t record_bytes = 2ll << 30;
 };
 
 constexpr int kSweepImporters = 8;   // most warps that fetch imports (a power of two)
@@ -52,6 +58,7 @@ constexpr int kSweepMaxWarps = 8;
 constexpr int kSweepStage = 4;         // records of a warp in shared memory
 constexpr int kSweepMaxSlots = 65535;
 constexpr int kSweepAhead = 24;        // records prefetched into the L2
+constexpr int kSweepRecordShare = 8;
 
 // bytes of shared memory beside the slots: block, epoch and the importers'
 // progress (128), the records on their way
@@ -83,8 +90,8 @@ struct SweepPlan {
 // inverse diagonal last in each row); es: bytes of a value (4 or 8).
 // level_hint (optional): a level per row in which every dependency has a lower
 // level.  Without blocks (ok() false) when a block cannot be made to fit, when
-// several blocks are needed and some row reads a later one, or when a kernel that
-// goes level by level costs less.
+// several blocks are needed and some row reads a later one, when the records would
+// take too much memory, or when a kernel that goes level by level costs less.
 SweepPlan build_sweep_plan(const int *rptr, const int *cind, const void *vals, int es, int n,
                            const SweepLimits &lim, const int *level_hint = nullptr);
 
