@@ -1183,7 +1183,8 @@ void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
 // LUflex::Solve / LU<T>::Solve (solver/lu.hpp:91-94, 30-33) by k_lu_chain (see
 // lu_chain.cuh).  k_dense_lu, one CTA and 32-row panels, left looking, solves FP32
 // (whose sums keep their order, see fixed_lanes; the chain took 64 us instead of 158
-// at n = 1013), the sequential-order mode and fixed-point shifts outside 0..31:
+// at n = 1013), FP64 systems of one panel, the sequential-order mode and fixed-point
+// shifts outside 0..31:
 // warps reduce a panel's rows against the solved part, lanes over the columns (one
 // thread a row in column order in the sequential-order mode), then a warp solves
 // the diagonal block.  Its factors are stored row by row.
@@ -1320,7 +1321,12 @@ void DevDenseLU::release() {
     L = U = Lb = Ub = dinv = nullptr;
 }
 
-static bool chain_takes(int vt, int bitL) { return vt == VT_F64 || (vt == VT_I32 && bitL >= 0 && bitL < 32); }
+// (FP64, one panel: there is nothing to hand to another CTA, and a step of the chain with
+// the next panel's product takes 190 cycles; n = 2 / 13 / 32 by the cluster 10.8 us, by
+// k_dense_lu 6.0 / 8.3 / 10.7)
+static bool chain_takes(int vt, int bitL, int n) {
+    return vt == VT_F64 ? n > 32 : vt == VT_I32 && bitL >= 0 && bitL < 32;
+}
 
 template <typename V>
 static void upload_lu(DevDenseLU &d, const int *Lrptr, const int *Lcind, const V *Lval, const int *Urptr,
@@ -1329,7 +1335,7 @@ static void upload_lu(DevDenseLU &d, const int *Lrptr, const int *Lcind, const V
     std::vector<V> dinv(std::max(n, 1), V(0));
     for (int i = 0; i < n; i++)  // dutri rows: D^-1 first, then the strict upper entries
         if (Urptr[i + 1] > Urptr[i]) dinv[i] = Uval[Urptr[i]];
-    if (chain_takes(d.vt, d.bitL)) {
+    if (chain_takes(d.vt, d.bitL, d.n)) {
         LuBlocks<V> B(n);
         B.dinv = dinv;
         for (int i = 0; i < n; i++) {
@@ -1401,7 +1407,7 @@ template <int VT, bool EXACT>
 static void launch_lu(Ctx &c, const DevDenseLU &LU, const void *in, void *out) {
     c.launches++;
     if constexpr (!EXACT && VT != VT_F32) {
-        if (chain_takes(VT, LU.bitL)) return launch_chain<VT>(c, LU, in, out);
+        if (chain_takes(VT, LU.bitL, LU.n)) return launch_chain<VT>(c, LU, in, out);
     }
     const size_t smem = (sizeof(acc_t<VT>) + sizeof(vt_t<VT>)) * (size_t)LU.n;
     k_dense_lu<VT, EXACT><<<1, kLuThreads, smem, c.stream>>>(LU.n, LU.L, LU.U, LU.dinv, LU.bitL, LU.bitU,
