@@ -346,7 +346,16 @@ struct FLuDesc {
 
 // LU<T>::Solve (lu.hpp:35-38) for every system and right-hand side: ltri forward
 // (x_i = in_i - sum_{j<i} l_ij x_j) then dutri backward
-// (x_i = (t_i - sum_{j>i} u_ij x_j) * dinv_i): FP64 one cluster each (lu_chain.cuh).
+// (x_i = (t_i - sum_{j>i} u_ij x_j) * dinv_i).
+//
+// FP64, up to a third as many systems as SMs (and more than one panel): one cluster for
+// each right-hand side (lu_chain.cuh).  Each reads the factors and holds four SMs (two CTAs of a cluster
+// share one), so with more systems the clusters run in several waves, while
+// k_flu_cta's one CTA a system, whatever the right-hand sides, still runs in one.
+// V-cycle of 8 / 32 / 48 / 64 / 96 / 152 systems of 68^2 to 80^2 by clusters and by CTAs,
+// us: one right-hand side 200 / 300 / 418 / 487 / 674 / 1,026 and 278 / 381 / 438 /
+// 499 / 617 / 825, two 235 / 439 / 596 / 761 / 1,078 / 1,612 and
+// 397 / 542 / 628 / 714 / 893 / 1,202.
 __global__ void __launch_bounds__(32 * kLuWarps, 1)
 k_flu_chain(const FLuDesc<double> *__restrict__ desc, int R, const double *__restrict__ Lcat,
             const double *__restrict__ Ucat, const double *__restrict__ dcat, unsigned *flags) {
@@ -357,9 +366,10 @@ k_flu_chain(const FLuDesc<double> *__restrict__ desc, int R, const double *__res
     lu_chain<VT_F64, true>(a, flags);
 }
 
-// FP32: one CTA per system, 32-row panels: warps reduce panel rows against the
-// solved part, warp 0 solves the diagonal block from registers.  An FP32 solve's
-// iterations follow the last bits, and the chain's sums have another order.
+// FP32, and FP64 with more systems: one CTA per system, 32-row panels: warps reduce
+// panel rows against the solved part, warp 0 solves the diagonal block from registers.
+// (An FP32 solve's iterations follow the last bits, and the chain's sums have another
+// order.)
 constexpr int kFLuThreads = 512;
 template <typename T, int R>
 __global__ void __launch_bounds__(kFLuThreads, 1)
@@ -901,6 +911,7 @@ class FpImpl : public BatchFpEngine::Base {
     FLuDesc<T> *d_lu = nullptr;
     int nlu = 0;
     size_t lu_smem = 0;
+    bool flu_chain = false;  // k_flu_chain, else k_flu_cta
     T *Lcat = nullptr, *Ucat = nullptr, *dcat = nullptr;
     DevCsr Af;
     std::vector<FTile> tiles_h;
@@ -966,6 +977,8 @@ class FpImpl : public BatchFpEngine::Base {
         std::vector<FLuDesc<T>> desc;
         std::vector<T> Lh, Uh, dh;
         size_t maxn = 0;
+        for (const BatchLUT<T> &lu : F.lu) maxn = std::max(maxn, (size_t)lu.n);
+        flu_chain = sizeof(T) == 8 && maxn > 32 && 3 * F.lu.size() <= (size_t)c.num_sms;
         for (const BatchLUT<T> &lu : F.lu) {
             FLuDesc<T> d{};
             d.n = lu.n;
@@ -974,28 +987,29 @@ class FpImpl : public BatchFpEngine::Base {
             d.d_off = (long long)dh.size();
             d.in = ee[lu.level] + (size_t)lu.offset * Rn;
             d.out = xx[lu.level] + (size_t)lu.offset * Rn;
-            if constexpr (sizeof(T) == 8) {
-                LuBlocks<T> B(lu.n);
-                for (int i = 0; i < lu.n; i++) {
-                    for (int j = 0; j < i; j++) B.L[B.lower(i, j)] = lu.L[(size_t)i * lu.n + j];
-                    for (int j = i + 1; j < lu.n; j++) B.U[B.upper(i, j)] = lu.U[(size_t)i * lu.n + j];
-                    B.dinv[i] = lu.dinv[i];
+            if (flu_chain) {
+                if constexpr (sizeof(T) == 8) {
+                    LuBlocks<T> B(lu.n);
+                    for (int i = 0; i < lu.n; i++) {
+                        for (int j = 0; j < i; j++) B.L[B.lower(i, j)] = lu.L[(size_t)i * lu.n + j];
+                        for (int j = i + 1; j < lu.n; j++) B.U[B.upper(i, j)] = lu.U[(size_t)i * lu.n + j];
+                        B.dinv[i] = lu.dinv[i];
+                    }
+                    B.scale_columns();
+                    Lh.insert(Lh.end(), B.L.begin(), B.L.end());
+                    Uh.insert(Uh.end(), B.U.begin(), B.U.end());
                 }
-                B.scale_columns();
-                Lh.insert(Lh.end(), B.L.begin(), B.L.end());
-                Uh.insert(Uh.end(), B.U.begin(), B.U.end());
             } else {
                 Lh.insert(Lh.end(), lu.L.begin(), lu.L.end());
                 Uh.insert(Uh.end(), lu.U.begin(), lu.U.end());
             }
             dh.insert(dh.end(), lu.dinv.begin(), lu.dinv.end());
-            maxn = std::max(maxn, (size_t)lu.n);
             desc.push_back(d);
         }
         nlu = (int)desc.size();
         lu_smem = 2 * sizeof(T) * maxn * Rn;
         if (lu_smem > 227 * 1024) throw CudaError{"a coarsest level is too large for the batched FP LU kernel"};
-        if (sizeof(T) == 8) lu_smem = ::sagb::lu_smem<VT_F64>((int)(maxn + 31) / 32).bytes;
+        if (flu_chain) lu_smem = ::sagb::lu_smem<VT_F64>((int)(maxn + 31) / 32).bytes;
         Lcat = dupload(Lh);
         Ucat = dupload(Uh);
         dcat = dupload(dh);
@@ -1019,13 +1033,11 @@ class FpImpl : public BatchFpEngine::Base {
         ascal = (T *)dmalloc(sizeof(T) * (size_t)S * Rn);
         info_d = (FInfo *)dmalloc(sizeof(FInfo));
         SAGB_CUDA(cudaMallocHost(&info_h, sizeof(FInfo)));
-        if constexpr (sizeof(T) == 8) {
+        if constexpr (sizeof(T) == 8)
             SAGB_CUDA(cudaFuncSetAttribute(k_flu_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLuChainSmem));
-        } else {
-            SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-            SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-            SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        }
+        SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        SAGB_CUDA(cudaFuncSetAttribute(k_flu_cta<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     }
 
     // LD in colour-row order: items {row, first entry, entries, 0}, the
@@ -1194,14 +1206,13 @@ class FpImpl : public BatchFpEngine::Base {
     void lu() {
         if (!nlu) return;
         if constexpr (sizeof(T) == 8)
-            launch_cluster(k_flu_chain, kLuCtas * nlu * Rn, 32 * kLuWarps, lu_smem, kLuCtas, (const FLuDesc<T> *)d_lu, Rn,
+            if (flu_chain) return launch_cluster(k_flu_chain, kLuCtas * nlu * Rn, 32 * kLuWarps, lu_smem, kLuCtas, (const FLuDesc<T> *)d_lu, Rn,
                            (const T *)Lcat, (const T *)Ucat, (const T *)dcat, c.d_flags);
-        else
-            by_r([&](auto RR) {
-                constexpr int R = decltype(RR)::value;
-                launch(k_flu_cta<T, R>, nlu, kFLuThreads, lu_smem, (const FLuDesc<T> *)d_lu, (const T *)Lcat,
-                       (const T *)Ucat, (const T *)dcat);
-            });
+        by_r([&](auto RR) {
+            constexpr int R = decltype(RR)::value;
+            launch(k_flu_cta<T, R>, nlu, kFLuThreads, lu_smem, (const FLuDesc<T> *)d_lu, (const T *)Lcat,
+                   (const T *)Ucat, (const T *)dcat);
+        });
     }
 
     // one-colour levels below the finest with their sweeps fused into the
