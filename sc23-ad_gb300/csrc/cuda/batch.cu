@@ -421,11 +421,6 @@ k_bcolour(int cnt, const int *__restrict__ rows, DBCsr LD, const int *__restrict
 // the cluster wrote them in an earlier colour.
 constexpr int kClusterCtas = 8;
 
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-
 template <int R, int G>
 __global__ void __launch_bounds__(kBThreads)
 k_bsweep_cluster(const int *__restrict__ gc_ptr, const int *__restrict__ cbound, const int *__restrict__ grows,
@@ -476,7 +471,7 @@ k_bsweep_cluster(const int *__restrict__ gc_ptr, const int *__restrict__ cbound,
                 if (any) atomicOr(flags, ST_OVERFLOW);
             }
         }
-        cluster_barrier();
+        cluster_sync_all();
     }
 }
 
@@ -639,7 +634,7 @@ k_bsweep_packed(const int *__restrict__ gc_ptr, const int *__restrict__ sw_ptr, 
         else nxt.ok = false;
 
         pk_row<R, G, true>(cur, ents, out, lane, row_sys, pflag, flags);
-        if (colour_end) cluster_barrier();
+        if (colour_end) cluster_sync_all();
         cur = nxt;
         k = nk;
         base = nbase;

@@ -193,16 +193,6 @@ struct EpochNet {
     int params() const { return H * I + H + H * H + H + O * H + O; }
 };
 
-__device__ __forceinline__ unsigned epoch_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void epoch_cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 __global__ void __launch_bounds__(kEpochThreads, 1)
 k_epoch(EpochNet N, const float *__restrict__ X, const float *__restrict__ T, const float *__restrict__ M,
         const int *__restrict__ perm, int n, int batch, const float *__restrict__ mu, const float *__restrict__ sd,
@@ -212,11 +202,10 @@ k_epoch(EpochNet N, const float *__restrict__ X, const float *__restrict__ T, co
     __shared__ float sh[32];
     __shared__ float s_tot;
     const int tid = threadIdx.x, I = N.I, H = N.H, O = N.O;
-    const unsigned rank = epoch_rank();
+    const unsigned rank = cluster_rank();
     unsigned other[kEpochCtas];  // this CTA's shared memory as the others see it: addresses in theirs
 #pragma unroll
-    for (int r = 0; r < kEpochCtas; r++)
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(other[r]) : "r"(smem_addr(sm)), "r"(r));
+    for (int r = 0; r < kEpochCtas; r++) other[r] = map_rank(smem_addr(sm), r);
     auto put = [&](int at, float v) {  // in every CTA
         sm[at] = v;
 #pragma unroll
@@ -255,9 +244,9 @@ k_epoch(EpochNet N, const float *__restrict__ X, const float *__restrict__ T, co
         a1 = m1[mine];
         a2 = m2[mine];
     }
-    epoch_cluster_sync();  // every CTA runs
+    cluster_sync_all();  // every CTA runs
     if (at >= 0) put(at, w);
-    epoch_cluster_sync();
+    cluster_sync_all();
 
     // activations, whole batch
     const int oX = N.acts(), oA1 = oX + batch * I, oA2 = oA1 + batch * H, oD1 = oA2 + batch * H, oD2 = oD1 + batch * H,
@@ -356,7 +345,7 @@ k_epoch(EpochNet N, const float *__restrict__ X, const float *__restrict__ T, co
         };
         backward(oDY, O, N.w3(), oA2, oD2, H);
         backward(oD2, H, N.w2(), oA1, oD1, H);
-        epoch_cluster_sync();
+        cluster_sync_all();
         // gradient and update of this thread's parameter
         if (at >= 0) {
             const int width = layer == 3 ? O : H, K = layer == 1 ? I : H;
@@ -384,7 +373,7 @@ k_epoch(EpochNet N, const float *__restrict__ X, const float *__restrict__ T, co
             const float esum = bsum(e);
             if (tid == 0) loss[s] = esum * inv;
         }
-        epoch_cluster_sync();
+        cluster_sync_all();
     }
     if (at >= 0) {
         p[mine] = w;
