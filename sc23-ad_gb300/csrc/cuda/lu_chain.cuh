@@ -388,13 +388,17 @@ __device__ __forceinline__ void lu_chain(const LuChain<VT> &a, unsigned *flags) 
             }
         }
     }
-    // no CTA leaves while a value may still be on its way into its shared memory
-    // (CTA 0 has waited for the sums)
+    // no CTA leaves while a value may still be on its way into its shared memory; CTA 0
+    // has waited for its blocks and sums, unless a wait ran out
     if (warp == kLuWarps - 1) {
         const unsigned long long t0 = globaltimer_ns();
-        for (int m = lane; m < 2 * npan; m += 32)
-            while (!mbar_try_wait(xbar + m, 0) && globaltimer_ns() - t0 <= kSpinLimitNs) {
-            }
+        auto arrived = [&](unsigned long long *bar) {
+            for (int m = lane; m < 2 * npan; m += 32)
+                while (!mbar_try_wait(bar + m, 0) && globaltimer_ns() - t0 <= kSpinLimitNs) {
+                }
+        };
+        arrived(xbar);
+        if (rank == 0 && *(volatile int *)&s_dead) arrived(ready);
     }
     __syncthreads();
     cluster_sync_all();
