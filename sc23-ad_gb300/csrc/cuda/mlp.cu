@@ -119,11 +119,13 @@ __global__ void k_mse(const float *__restrict__ Y, const float *__restrict__ T, 
     if (threadIdx.x == 0) *loss = esum * inv;
 }
 
-// Adam (Kingma & Ba 2015) with bias correction; t is the 1-based step count.
+// Adam (Kingma & Ba 2015) with bias correction; t is the 1-based step count.  The
+// multiply-adds are written out: left to the compiler, each kernel fuses either product
+// of a moment, and the weights after some steps depend on which.
 __device__ __forceinline__ float adam_step(float w, float gi, float &m1, float &m2, float lr, float beta1, float beta2,
                                            float eps, float bc1, float bc2) {
-    m1 = beta1 * m1 + (1.f - beta1) * gi;
-    m2 = beta2 * m2 + (1.f - beta2) * gi * gi;
+    m1 = __fmaf_rn(1.f - beta1, gi, __fmul_rn(beta1, m1));
+    m2 = __fmaf_rn(__fmul_rn(1.f - beta2, gi), gi, __fmul_rn(beta2, m2));
     const float mh = m1 / bc1, vh = m2 / bc2;
     return w - lr * mh / (sqrtf(vh) + eps);
 }
