@@ -355,7 +355,7 @@ __global__ void k_v0_fp(int n, const double *__restrict__ r, const FScal<T> *__r
         V0[i] = (T)__dmul_rn(r[i], e_inv);
 }
 
-template <typename T, int G>
+template <typename T, int G, int V>  // V: DevCsr::sums
 __global__ void __launch_bounds__(kRedThreads)
 k_spmv_dot_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, const T *__restrict__ val,
               const T *__restrict__ z, T *__restrict__ w, const T *__restrict__ v0, T *partials,
@@ -364,7 +364,7 @@ k_spmv_dot_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind,
     const long long tid = (long long)blockIdx.x * kRedThreads + threadIdx.x;
     const int row = (int)(tid / G), lane = (int)(tid % G);
     T a = 0;
-    if (row < n) a = row_part<G>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, z);
+    if (row < n) a = row_sums<G, V>(__ldg(rptr + row), __ldg(rptr + row + 1), lane, cind, val, z);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) a += shfl_xor(a, o);
     T d = 0;
@@ -822,11 +822,22 @@ class FpSolver : public SolverBase {
                     k_givens_fp<T, true><<<1, 1, 0, c_.stream>>>(j, m, H_, cs_, sn_, e_, sc_, info_d_, c_.d_flags);
                     c_.launches += 2 * j + 4;
                 } else {
-                    by_group(A_->lanes ? A_->lanes : A_->group, [&](auto G) {
+                    // (FP32: by all the lanes that its sums stand for, so that the dot product
+                    // keeps its order too)
+                    constexpr bool kF32 = std::is_same<T, float>::value;
+                    by_group(kF32 ? A_->group * A_->sums : A_->group, [&](auto G) {
                         const long long thr = (long long)N * G.value;
                         const int blocks = (int)((thr + kRedThreads - 1) / kRedThreads);
-                        k_spmv_dot_fp<T, G.value><<<blocks, kRedThreads, 0, c_.stream>>>(
-                            N, A_->rptr, A_->cind, (const T *)A_->val, zj, w, V_, partials_, counter_, Hj);
+                        auto run = [&](auto kern) {
+                            kern<<<blocks, kRedThreads, 0, c_.stream>>>(N, A_->rptr, A_->cind, (const T *)A_->val, zj, w, V_,
+                                                                        partials_, counter_, Hj);
+                        };
+                        if constexpr (!kF32) {
+                            if constexpr (G.value <= 16)
+                                if (A_->sums == 2) return run(k_spmv_dot_fp<T, G.value, 2>);
+                            if (A_->sums == SUMS_HALVES) return run(k_spmv_dot_fp<T, G.value, SUMS_HALVES>);
+                        }
+                        run(k_spmv_dot_fp<T, G.value, 1>);
                     });
                     for (int k = 0; k < j; k++)
                         k_mgs_fp<T, false><<<gb, kRedThreads, 0, c_.stream>>>(N, k, j, m, V_, w, H_, partials_,

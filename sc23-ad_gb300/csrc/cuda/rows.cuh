@@ -3,7 +3,8 @@
 // Bound by memory latency and, with one lane a row, by the L1 cache (each load
 // of a warp touches as many lines as rows): four entries a lane are in flight,
 // the last one to three in one predicated round, and the kernels stay at 32
-// registers, so that an SM holds all its threads.  Poisson 127^3 (FP64, 2.05 M
+// registers (FP32 with eight sums a lane: 40), so that an SM holds all its threads.
+// Poisson 127^3 (FP64, 2.05 M
 // rows of 7 entries), one lane a row: 39.6 us = 5.4 TB/s; one entry at a time
 // and four lanes a row, 131 us.  Copying the entries of 256 rows into shared
 // memory first was slower: 42 us, with the next 256 rows' copy behind the sums
@@ -11,6 +12,7 @@
 #pragma once
 #include <type_traits>
 
+#include "../sagb_internal.hpp"
 #include "common.cuh"
 
 namespace sagb {
@@ -28,11 +30,12 @@ __device__ __forceinline__ float row_add(float a, float v, float x) {
     return EXACT ? __fadd_rn(a, __fmul_rn(v, x)) : a + v * x;
 }
 
-// entries a + lane, a + lane + G, ... below b
-template <int G, bool EXACT = false, typename V>
+// entries a + lane, a + lane + G, ... below b, in S sums in turn
+template <int G, bool EXACT = false, int S = 1, typename V>
 __device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__restrict__ cind, const V *__restrict__ val,
                                          const V *__restrict__ x) {
-    std::conditional_t<std::is_same<V, int>::value, long long, V> acc = 0;
+    static_assert(S == 1 || S == 2, "one sum or two");
+    std::conditional_t<std::is_same<V, int>::value, long long, V> acc[S] = {};
     int j = a + lane;
     for (; j + 3 * G < b; j += 4 * G) {
         int c[4];
@@ -45,7 +48,7 @@ __device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__re
 #pragma unroll
         for (int q = 0; q < 4; q++) xv[q] = __ldg(x + c[q]);
 #pragma unroll
-        for (int q = 0; q < 4; q++) acc = row_add<EXACT>(acc, v[q], xv[q]);
+        for (int q = 0; q < 4; q++) acc[q % S] = row_add<EXACT>(acc[q % S], v[q], xv[q]);
     }
     if (j + G < b) {
         const bool third = j + 2 * G < b;
@@ -59,12 +62,13 @@ __device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__re
 #pragma unroll
         for (int q = 0; q < 3; q++) xv[q] = q < 2 || third ? __ldg(x + c[q]) : V(0);
 #pragma unroll
-        for (int q = 0; q < 2; q++) acc = row_add<EXACT>(acc, v[q], xv[q]);
-        if (third) acc = row_add<EXACT>(acc, v[2], xv[2]);
+        for (int q = 0; q < 2; q++) acc[q % S] = row_add<EXACT>(acc[q % S], v[q], xv[q]);
+        if (third) acc[0] = row_add<EXACT>(acc[0], v[2], xv[2]);
     } else if (j < b) {
-        acc = row_add<EXACT>(acc, __ldg(val + j), __ldg(x + __ldg(cind + j)));
+        acc[0] = row_add<EXACT>(acc[0], __ldg(val + j), __ldg(x + __ldg(cind + j)));
     }
-    return acc;
+    if constexpr (S == 2) return acc[0] + acc[1];
+    else return acc[0];
 }
 
 // The sum that G * V lanes a row give, taken by G: lane g keeps the V partial sums
@@ -95,6 +99,33 @@ __device__ __forceinline__ T row_part_of(int a, int b, int lane, const int *__re
 #pragma unroll
         for (int v = 0; v < o; v++) acc[v] += acc[v + o];
     return acc[0];
+}
+
+// FP64: the lane's entries in two sums, so that a row is as exact as by about as many
+// lanes as it has entries (a running sum past a large diagonal was up to 1.4 times as
+// far off).  HALVES: the first half and one more (the diagonal of a symmetric row is its
+// last), then the rest; else alternating, for lanes with few entries.  An FP64 addition
+// keeps a scheduler busy for 64 cycles, so this costs one: Poisson 127^3 with one sum 36
+// us, two 37, four 54, the eight of the lanes before 58.
+template <int G, bool HALVES>
+__device__ __forceinline__ double row_pair(int a, int b, int lane, const int *__restrict__ cind, const double *__restrict__ val,
+                                           const double *__restrict__ x) {
+    if constexpr (HALVES) {
+        const int mid = min(b, a + ((b - a + G - 1) / G / 2 + 1) * G);
+        const double first = row_part<G>(a, mid, lane, cind, val, x);
+        return first + row_part<G>(mid, b, lane, cind, val, x);
+    } else {
+        return row_part<G, false, 2>(a, b, lane, cind, val, x);
+    }
+}
+
+// the lane's part of an FP row by DevCsr::sums
+template <int G, int V, typename T>
+__device__ __forceinline__ T row_sums(int a, int b, int lane, const int *__restrict__ cind, const T *__restrict__ val,
+                                      const T *__restrict__ x) {
+    if constexpr (V == 1) return row_part<G>(a, b, lane, cind, val, x);
+    else if constexpr (std::is_same<T, double>::value) return row_pair<G, V == SUMS_HALVES>(a, b, lane, cind, val, x);
+    else return row_part_of<G, V>(a, b, lane, cind, val, x);
 }
 
 }  // namespace sagb

@@ -59,6 +59,20 @@ DevCsr upload_csr_i32(const CsrI &A) {
     return d;
 }
 
+// FP32 rows are summed in the order that pick_group lanes give, however many take them
+// (row_part_of); FP64 rows by fewer lanes than those in two sums a lane (row_pair).
+static void fp_lanes(DevCsr &d, const int *rptr) {
+    const double avg = d.n ? (double)d.nnz / d.n : 1.0;
+    const int as = pick_group(avg), longest = longest_row(rptr, d.n);
+    if (d.vt == VT_F32) {
+        d.group = std::max(spmv_lanes(d.n, d.nnz, longest, as), as / 8);
+        d.sums = as / d.group;
+    } else {
+        d.group = spmv_lanes(d.n, d.nnz, longest);
+        d.sums = d.group >= as ? 1 : avg >= 4.5 * d.group ? SUMS_HALVES : 2;
+    }
+}
+
 template <typename T>
 DevCsr upload_csr_fp(const CsrT<T> &A) {
     DevCsr d;
@@ -69,10 +83,7 @@ DevCsr upload_csr_fp(const CsrT<T> &A) {
     d.rptr = dupload(A.rptr);
     d.cind = A.cind.empty() ? (int *)dmalloc(16) : dupload(A.cind);
     d.val = A.val.empty() ? dmalloc(16) : (void *)dupload(A.val);
-    // FP32: the row's sum as by d.lanes lanes (see row_part_of)
-    if (d.vt == VT_F32) d.lanes = pick_group(A.n ? (double)d.nnz / A.n : 1.0);
-    d.group = spmv_lanes(A.n, d.nnz, longest_row(A.rptr.data(), A.n), d.lanes ? d.lanes : 32);
-    if (d.lanes) d.group = std::max(d.group, d.lanes / 8);
+    fp_lanes(d, A.rptr.data());
     return d;
 }
 template DevCsr upload_csr_fp<double>(const CsrT<double> &);
@@ -87,7 +98,7 @@ DevCsr upload_csr_f64(const CsrD &A) {
     d.rptr = dupload(A.rptr);
     d.cind = dupload(A.cind);
     d.val = dupload(A.val);
-    d.group = spmv_lanes(A.n, d.nnz, longest_row(A.rptr.data(), A.n));
+    fp_lanes(d, A.rptr.data());
     return d;
 }
 
@@ -131,7 +142,7 @@ k_spmv_i32(int n, const int *__restrict__ rptr, const int *__restrict__ cind, co
     if (lane == 0 && row < n && spmv_store<int, MODE>(acc, row, y, z, bit)) atomicOr(flags, ST_OVERFLOW);
 }
 
-template <typename T, int G, int V, int MODE, bool EXACT>  // V: see row_part_of
+template <typename T, int G, int V, int MODE, bool EXACT>  // V: DevCsr::sums
 __global__ void __launch_bounds__(kSpmvThreads)
 k_spmv_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, const T *__restrict__ val,
           const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ z) {
@@ -141,8 +152,8 @@ k_spmv_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, con
     T acc = 0;
     if (row < n) {
         const int a = __ldg(rptr + row), b = __ldg(rptr + row + 1);
-        if constexpr (V > 1) acc = row_part_of<G, V>(a, b, lane, cind, val, x);
-        else acc = row_part<G, EXACT>(a, b, lane, cind, val, x);
+        if constexpr (V == 1) acc = row_part<G, EXACT>(a, b, lane, cind, val, x);
+        else acc = row_sums<G, V>(a, b, lane, cind, val, x);
     }
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) acc += shfl_xor(acc, o);
@@ -184,16 +195,18 @@ static void dispatch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mod
     if (c.fp_exact) return launch_fp<T, 1, true>(c, A, x, y, mode, z);
     auto by_v = [&](auto G) {
         constexpr int g = decltype(G)::value;
-        if constexpr (std::is_same<T, float>::value && g <= 16) {
-            if (A.lanes == 2 * g) return launch_fp<T, g, false, 2>(c, A, x, y, mode, z);
+        if (A.sums == 1) return launch_fp<T, g, false, 1>(c, A, x, y, mode, z);
+        if constexpr (g <= 16)
+            if (A.sums == 2) return launch_fp<T, g, false, 2>(c, A, x, y, mode, z);
+        if constexpr (std::is_same<T, double>::value) {
+            if (A.sums == SUMS_HALVES) return launch_fp<T, g, false, SUMS_HALVES>(c, A, x, y, mode, z);
+        } else {
             if constexpr (g <= 8)
-                if (A.lanes == 4 * g) return launch_fp<T, g, false, 4>(c, A, x, y, mode, z);
+                if (A.sums == 4) return launch_fp<T, g, false, 4>(c, A, x, y, mode, z);
             if constexpr (g <= 4)
-                if (A.lanes == 8 * g) return launch_fp<T, g, false, 8>(c, A, x, y, mode, z);
+                if (A.sums == 8) return launch_fp<T, g, false, 8>(c, A, x, y, mode, z);
         }
-        // (any other sum would have another order)
-        if (A.lanes && A.lanes != g) throw CudaError{"no SpMV kernel for this number of lanes"};
-        launch_fp<T, g, false>(c, A, x, y, mode, z);
+        throw CudaError{"no SpMV kernel for these lanes"};  // (any other sum would have another order)
     };
     switch (A.group) {
         case 1: return by_v(std::integral_constant<int, 1>());
