@@ -93,13 +93,11 @@ __device__ __forceinline__ void st_async_u64(unsigned addr, unsigned long long v
 template <typename T>
 __device__ __forceinline__ unsigned long long bits_of(T v) {
     if constexpr (std::is_same<T, double>::value) return (unsigned long long)__double_as_longlong(v);
-    else if constexpr (std::is_same<T, float>::value) return (unsigned long long)__float_as_uint(v);
     else return (unsigned long long)v;
 }
 template <typename T>
 __device__ __forceinline__ T of_bits(unsigned long long v) {
     if constexpr (std::is_same<T, double>::value) return __longlong_as_double((long long)v);
-    else if constexpr (std::is_same<T, float>::value) return __uint_as_float((unsigned)v);
     else return (T)v;
 }
 

@@ -568,7 +568,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 
 constexpr int kSweepThreads = 32 * (kSweepMaxWarps + kSweepImporters);
 
-// N: lanes that one stands for, each with a sum of its own (FP32, see fixed_lanes)
+// N: lanes that one stands for, each with a sum of its own (FP32, see fixed_order)
 template <int VT, bool EXACT, int LG, int E, int N = 1>
 __global__ void __launch_bounds__(kSweepThreads, 1)
 k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
@@ -714,7 +714,7 @@ k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
         // the record kSweepStage - 1 ahead goes where the last one was
         copy(to);
         to = to == (kSweepStage - 1) * RB ? 0 : to + RB;
-        if (odd) {  // two records' lines
+        if (odd) {  // two records are 8 Q lines, at most one a lane: of four pairs' 40 or 48, the first 32
             if (lane < 8 * Q) prefetch_l2(ahead);
             ahead += 2 * RB;
         }
@@ -742,8 +742,8 @@ k_sweep(SweepArgs a, const void *in_, void *out_, unsigned *flags) {
             s = sn[0];
         } else {
             s = t;
-            acc_t<VT> s2 = 0;  // (two chains where the order is free)
-            if constexpr (VT == VT_F64 && LG == 0) s = fresh ? own : t;  // one lane a row: its sum in its order
+            acc_t<VT> s2 = 0;  // (two chains a record where the order is free)
+            if constexpr (VT == VT_F64 && LG == 0) s = fresh ? own : t;  // one lane a row: it starts from the input
 #pragma unroll
             for (int h = 0; h < 2 * E; h++) {
                 const uint4 &v = r[1 + h / 2];
@@ -881,7 +881,7 @@ static int tri_lanes(const Ctx &c, const TriSource &t, int vt) {
     return pow2_at_least((t.n ? ((double)t.rptr[t.n] - t.n) / t.n : 0.0) / kRowShare);
 }
 
-// Lanes a row where its sum has one order: one in the sequential-order mode.  FP32
+// Whether a row's sum has one order: in the sequential-order mode, and in FP32.  FP32
 // solves converge in a number of iterations that follows the last bits of their
 // V-cycles, so an FP32 row is summed by all kernels as by tri_lanes lanes, which
 // depend on its triangle alone: lane g takes entries g, g + G, ... in their order,
@@ -1182,7 +1182,7 @@ void trsv_noalloc(Ctx &c, const DevTri &T, const void *in, void *out) {
 //
 // LUflex::Solve / LU<T>::Solve (solver/lu.hpp:91-94, 30-33) by k_lu_chain (see
 // lu_chain.cuh).  k_dense_lu, one CTA and 32-row panels, left looking, solves FP32
-// (whose sums keep their order, see fixed_lanes; the chain took 64 us instead of 158
+// (whose sums keep their order, see fixed_order; the chain took 64 us instead of 158
 // at n = 1013), FP64 systems of one panel, the sequential-order mode and fixed-point
 // shifts outside 0..31:
 // warps reduce a panel's rows against the solved part, lanes over the columns (one
