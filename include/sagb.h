@@ -234,7 +234,8 @@ int sa_amg_sweep(sa_ctx ctx, sa_amg M, int level, const void *in, void *out);
  * framework's caching allocator, a fixed pool), or they cannot afford the
  * device-wide synchronisation that allocating and freeing imply.  in and out
  * must be device buffers.  Levels whose vectors take at most 150 KiB sweep in the
- * context's own scratch, like sa_amg_sweep.  The scratch of larger ones comes
+ * context's own scratch, like sa_amg_sweep (a captured call uses it whenever its
+ * graph runs: in order with the context's other calls).  The scratch of larger ones comes
  * from a static device array sized for 262,144 rows (4 MiB, held by every GPU
  * that loads the library until the process exits); a level with more rows is
  * rejected with SA_ERR_ARG.  The first of their calls on a device looks up that
