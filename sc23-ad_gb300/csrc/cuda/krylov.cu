@@ -836,6 +836,8 @@ class FpSolver : public SolverBase {
                             if constexpr (G.value <= 16)
                                 if (A_->sums == 2) return run(k_spmv_dot_fp<T, G.value, 2>);
                             if (A_->sums == SUMS_HALVES) return run(k_spmv_dot_fp<T, G.value, SUMS_HALVES>);
+                            if constexpr (G.value == 1)
+                                if (A_->sums == SUMS_PAIRS) return run(k_spmv_dot_fp<T, G.value, SUMS_PAIRS>);
                         }
                         run(k_spmv_dot_fp<T, G.value, 1>);
                     });

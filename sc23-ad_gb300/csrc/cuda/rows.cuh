@@ -30,8 +30,9 @@ __device__ __forceinline__ float row_add(float a, float v, float x) {
     return EXACT ? __fadd_rn(a, __fmul_rn(v, x)) : a + v * x;
 }
 
-// entries a + lane, a + lane + G, ... below b, in S sums in turn
-template <int G, bool EXACT = false, int S = 1, typename V>
+// entries a + lane, a + lane + G, ... below b, in S sums in turn; SINGLY: the last one to
+// three one by one
+template <int G, bool EXACT = false, int S = 1, bool SINGLY = false, typename V>
 __device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__restrict__ cind, const V *__restrict__ val,
                                          const V *__restrict__ x) {
     static_assert(S == 1 || S == 2, "one sum or two");
@@ -50,7 +51,10 @@ __device__ __forceinline__ auto row_part(int a, int b, int lane, const int *__re
 #pragma unroll
         for (int q = 0; q < 4; q++) acc[q % S] = row_add<EXACT>(acc[q % S], v[q], xv[q]);
     }
-    if (j + G < b) {
+    if constexpr (SINGLY) {
+        static_assert(S == 1, "one sum");
+        for (; j < b; j += G) acc[0] = row_add<EXACT>(acc[0], __ldg(val + j), __ldg(x + __ldg(cind + j)));
+    } else if (j + G < b) {
         const bool third = j + 2 * G < b;
         int c[3];
         V v[3], xv[3];
@@ -119,12 +123,46 @@ __device__ __forceinline__ double row_pair(int a, int b, int lane, const int *__
     }
 }
 
+// FP64, about as many lanes as entries: one or two entries a lane.  An addition keeps a
+// scheduler busy for 64 cycles also where few lanes of the warp take it, so the lanes take
+// their last entries one by one, whatever number of them each has.  (32 lanes, one row a
+// warp: only where it has no more than two a lane.)  12,000 rows of 9 entries 5.2 -> 4.2
+// us, of 0 to 14 5.1 -> 4.2, 1.5 M rows of 0 to 2 entries 12.4 -> 10.3.
+template <int G>
+__device__ __forceinline__ double row_few(int a, int b, int lane, const int *__restrict__ cind, const double *__restrict__ val,
+                                          const double *__restrict__ x) {
+    if constexpr (G == 32)
+        if (b - a > 2 * G) return row_part<G>(a, b, lane, cind, val, x);
+    return row_part<G, false, 1, true>(a, b, lane, cind, val, x);
+}
+
+// FP64, one lane and few entries a row, as in interpolations (rows of one next to rows of
+// four): the two sums' entries pair by pair, for the same reason.  1.5 M rows of 0 to 4
+// entries 26.8 -> 17.4 us, of 0 to 6 27.2 -> 22.7, but of 0 to 8 38.9 -> 43.2 and of 3
+// each 14.5 -> 17.5: only below 2.6 entries a row.
+__device__ __forceinline__ double row_two(int a, int b, const int *__restrict__ cind, const double *__restrict__ val,
+                                          const double *__restrict__ x) {
+    double first = 0, second = 0;
+    for (int j = a; j < b; j += 2) {
+        const bool two = j + 1 < b;
+        const int c0 = __ldg(cind + j), c1 = two ? __ldg(cind + j + 1) : 0;
+        const double v0 = __ldg(val + j), v1 = two ? __ldg(val + j + 1) : 0.0;
+        const double x0 = __ldg(x + c0), x1 = two ? __ldg(x + c1) : 0.0;
+        first += v0 * x0;
+        if (two) second += v1 * x1;
+    }
+    return first + second;
+}
+
 // the lane's part of an FP row by DevCsr::sums
 template <int G, int V, typename T>
 __device__ __forceinline__ T row_sums(int a, int b, int lane, const int *__restrict__ cind, const T *__restrict__ val,
                                       const T *__restrict__ x) {
-    if constexpr (V == 1) return row_part<G>(a, b, lane, cind, val, x);
-    else if constexpr (std::is_same<T, double>::value) return row_pair<G, V == SUMS_HALVES>(a, b, lane, cind, val, x);
+    if constexpr (std::is_same<T, double>::value) {
+        if constexpr (V == 1) return row_few<G>(a, b, lane, cind, val, x);
+        else if constexpr (V == SUMS_PAIRS) return row_two(a, b, cind, val, x);
+        else return row_pair<G, V == SUMS_HALVES>(a, b, lane, cind, val, x);
+    } else if constexpr (V == 1) return row_part<G>(a, b, lane, cind, val, x);
     else return row_part_of<G, V>(a, b, lane, cind, val, x);
 }
 

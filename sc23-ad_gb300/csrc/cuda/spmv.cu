@@ -69,7 +69,7 @@ static void fp_lanes(DevCsr &d, const int *rptr) {
         d.sums = as / d.group;
     } else {
         d.group = spmv_lanes(d.n, d.nnz, longest);
-        d.sums = d.group >= as ? 1 : avg >= 4.5 * d.group ? SUMS_HALVES : 2;
+        d.sums = d.group >= as ? 1 : avg >= 4.5 * d.group ? SUMS_HALVES : d.group == 1 && avg < 2.6 ? SUMS_PAIRS : 2;
     }
 }
 
@@ -152,7 +152,7 @@ k_spmv_fp(int n, const int *__restrict__ rptr, const int *__restrict__ cind, con
     T acc = 0;
     if (row < n) {
         const int a = __ldg(rptr + row), b = __ldg(rptr + row + 1);
-        if constexpr (V == 1) acc = row_part<G, EXACT>(a, b, lane, cind, val, x);
+        if constexpr (EXACT) acc = row_part<G, EXACT>(a, b, lane, cind, val, x);
         else acc = row_sums<G, V>(a, b, lane, cind, val, x);
     }
 #pragma unroll
@@ -200,6 +200,8 @@ static void dispatch_fp(Ctx &c, const DevCsr &A, const void *x, void *y, int mod
             if (A.sums == 2) return launch_fp<T, g, false, 2>(c, A, x, y, mode, z);
         if constexpr (std::is_same<T, double>::value) {
             if (A.sums == SUMS_HALVES) return launch_fp<T, g, false, SUMS_HALVES>(c, A, x, y, mode, z);
+            if constexpr (g == 1)
+                if (A.sums == SUMS_PAIRS) return launch_fp<T, g, false, SUMS_PAIRS>(c, A, x, y, mode, z);
         } else {
             if constexpr (g <= 8)
                 if (A.sums == 4) return launch_fp<T, g, false, 4>(c, A, x, y, mode, z);

@@ -84,14 +84,14 @@ T *dupload(const std::vector<T> &v) {
 }
 
 // ------------------------------------------------------------------ matrices
-constexpr int SUMS_HALVES = 0;
+constexpr int SUMS_HALVES = 0, SUMS_PAIRS = -1;
 struct DevCsr {
     int n = 0, m = 0;
     int64_t nnz = 0;
     int bit = 0;
     int vt = VT_I32;
     int group = 1;  // lanes per row in the SpMV kernel
-    int sums = 1;   // FP: sums of a lane (cuda/rows.cuh): FP32 1, 2, 4 or 8, FP64 1, 2 or SUMS_HALVES
+    int sums = 1;   // FP: sums of a lane (cuda/rows.cuh): FP32 1, 2, 4 or 8, FP64 1, 2, SUMS_HALVES or SUMS_PAIRS
     int *rptr = nullptr, *cind = nullptr;
     void *val = nullptr;
     void release();
