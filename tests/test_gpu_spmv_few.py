@@ -20,6 +20,7 @@ ld = np.longdouble
     (sagb.MAT_F64, np.float64, 12001, 18, 8),
     (sagb.MAT_F64, np.float64, 2003, 41, 16),
     (sagb.MAT_F64, np.float64, 2003, 90, 32),  # rows on both sides of two entries a lane
+    (sagb.MAT_F32, np.float32, 20001, 440, 32),  # all lanes of the order
 ])
 def test_order(kind, dtype, n, most, G):
     rng = np.random.default_rng(most)
